@@ -22,6 +22,7 @@
 // st_b200_mlp_error) and the kernel drains and returns, freeing its tensor memory.
 #include <cstdint>
 #include <cstdio>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -299,13 +300,67 @@ __global__ void k_mse(int rows, int cols, const float *y, const float *t, long l
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
 }
 
-// db[c] = sum over rows of dz[r][c] (one thread per column; rows strided by cols)
-__global__ void k_colsum(int rows, int cols, const __nv_bfloat16 *dz, float *db) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += __bfloat162float(dz[(long long)r * cols + c]);
-    db[c] = s;
+// db[c] = sum over rows of dz[r][c].  Bound by reading dz once (L2-resident behind the product
+// that wrote it).  A cluster of kSumCluster CTAs owns kSumCols columns, its CTAs splitting the
+// rows: a thread adds every 512th row of its eight columns (16-byte loads), the CTA folds its
+// 64 row lanes in shared memory and the cluster's first CTA adds the others' sums read through
+// distributed shared memory, always in the same order (no atomics, no cleared output).  32
+// columns a cluster keep 64 bytes of a row together and give 64 CTAs at 256 columns.
+// One thread per column (2 blocks at 256 columns, a serial chain over the rows) took 926 us at
+// 16,384 rows, two thirds of a gradient pass, which fell from 4.81 to 2.31 ms with this kernel.
+constexpr int kSumCols = 32, kSumCluster = 8, kSumThreads = 256;
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
+    k_colsum(int rows, int cols, const __nv_bfloat16 *dz, float *db) {
+    namespace cg = cooperative_groups;
+    constexpr int kLanes = kSumThreads / (kSumCols / 8);  // row lanes of a CTA
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ float part[kLanes][kSumCols + 1];
+    __shared__ float sum[kSumCols];
+    const int q = threadIdx.x % (kSumCols / 8), lane = threadIdx.x / (kSumCols / 8);
+    const int c0 = int(blockIdx.x / kSumCluster) * kSumCols + 8 * q;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    // whole 16-byte chunks of an aligned matrix; single values otherwise
+    const bool wide = cols % 8 == 0 && (reinterpret_cast<uintptr_t>(dz) & 15) == 0;
+    if (c0 < cols) {
+#pragma unroll 4
+        for (int r = int(cluster.block_rank()) * kLanes + lane; r < rows; r += kSumCluster * kLanes) {
+            const __nv_bfloat16 *p = dz + (long long)r * cols + c0;
+            if (wide) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(p);
+                const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[2 * i] += __uint_as_float(h[i] << 16);
+                    s[2 * i + 1] += __uint_as_float(h[i] & 0xffff0000u);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (c0 + i < cols) s[i] += __bfloat162float(p[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[lane][8 * q + i] = s[i];
+    __syncthreads();
+    for (int o = kLanes / 2; o >= kSumThreads / kSumCols; o >>= 1) {
+        for (int k = threadIdx.x; k < o * kSumCols; k += kSumThreads)
+            part[k / kSumCols][k % kSumCols] += part[k / kSumCols + o][k % kSumCols];
+        __syncthreads();
+    }
+    if (threadIdx.x < kSumCols) {
+        float t = 0.f;
+        for (int k = 0; k < kSumThreads / kSumCols; ++k) t += part[k][threadIdx.x];
+        sum[threadIdx.x] = t;
+    }
+    cluster.sync();
+    const int c = int(blockIdx.x / kSumCluster) * kSumCols + int(threadIdx.x);
+    if (cluster.block_rank() == 0 && threadIdx.x < kSumCols && c < cols) {
+        float t = 0.f;
+        for (int b = 0; b < kSumCluster; ++b) t += *cluster.map_shared_rank(&sum[threadIdx.x], b);
+        db[c] = t;
+    }
+    cluster.sync();  // the other CTAs' sums stay until they are read
 }
 
 // Adam (Kingma & Ba 2015) on float master weights, with the bf16 copy the GEMMs read
@@ -804,7 +859,8 @@ int st_b200_mlp_mse(int rows, int cols, const float *y, const float *target, lon
 
 int st_b200_mlp_colsum(int rows, int cols, const void *dz, float *db, void *stream) {
     if (rows <= 0 || cols <= 0 || !dz || !db) return -1;
-    k_colsum<<<(cols + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const unsigned chunks = unsigned((cols + (long long)kSumCols - 1) / kSumCols);
+    k_colsum<<<chunks * kSumCluster, kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         rows, cols, static_cast<const __nv_bfloat16 *>(dz), db);
     return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }

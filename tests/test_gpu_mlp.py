@@ -89,6 +89,23 @@ def test_gemm_matches_host(mlp_env, case):
     assert err <= tol, (err, tol)
 
 
+@pytest.mark.parametrize("rows,cols,offset", [(1, 1, 0), (63, 7, 1), (512, 32, 0), (513, 33, 0), (2049, 256, 0),
+                                              (1000, 1024, 3), (16384, 40, 0)])
+def test_colsum_matches_host(mlp_env, rows, cols, offset):
+    """Column sums at the edges of the kernel's 32 columns x 512 row lanes, with wide and with
+    element loads (an offset leaves the matrix unaligned), against float64 sums of the same bf16
+    values: at most 65 + 16 float additions of a column's values, each rounding the partial sum
+    (|partial| <= the column's absolute sum) by 2^-24."""
+    torch, net = mlp_env
+    g = torch.Generator(device="cpu").manual_seed(rows + cols)
+    flat = torch.randn(rows * cols + offset, generator=g).to(torch.bfloat16).cuda()
+    dz = flat[offset:].view(rows, cols)
+    db = torch.full((cols,), 7.0, device="cuda")
+    assert net.api.lib.st_b200_mlp_colsum(rows, cols, dz.data_ptr(), db.data_ptr(), net._s()) == 1
+    want, tol = dz.double().sum(0), dz.double().abs().sum(0) * (rows / 512 + 82) * 2.0 ** -24
+    assert bool(((db.double() - want).abs() <= tol).all())
+
+
 def test_network_gradients_match_oracle(product):
     import torch
     import mlp_oracle
