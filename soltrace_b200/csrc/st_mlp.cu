@@ -6,23 +6,26 @@
 // per-source flux map) makes its training data and measures its error.  It has no counterpart in the
 // reference, which traces every ray.
 //
-// One GEMM kernel does every layer's work, forward and backward:
+// One product does every layer's work, forward and backward:
 //     C[M x N] = epilogue(A[M x K] B[N x K]^T)
 // with A(m, k) = A[m lam + k lak] and B(n, k) = B[n lbn + k lbk] (bf16), so the backward
-// products (dX = dZ W, dW = dZ^T X) read their operands in place through strides.  A CTA of
-// 128 threads owns a 128 x BN tile of C: per 64-wide slice of K it stages the A and B tiles in
-// shared memory in the K-major, unswizzled core-matrix layout the tensor cores read (8 rows x
-// 16 bytes per core matrix), one elected thread issues four tcgen05.mma (K = 16 each) into the
-// tile's FP32 accumulator in tensor memory and commits them to an mbarrier, and after the last
-// slice the four warps read the accumulator back (tcgen05.ld, one row per thread) and apply
-// the epilogue.  Split-K: gridDim.z CTAs share a tile's K range and add their partial sums
-// (EPI_F32_ADD).
+// products (dX = dZ W, dW = dZ^T X) read their operands in place through strides.  Split-K: several
+// CTAs share a tile's K range and add their partial sums (EPI_F32_ADD).  Two kernels:
+//   k_mlp_gemm_tma, a warp-specialised TMA pipeline, for operands TMA can address (every layer
+//     of a network whose widths are multiples of 8);
+//   k_mlp_gemm for any strides: a CTA of 128 threads owns a 128 x BN tile of C; per 64-wide slice
+//     of K it stages the A and B tiles in shared memory in the K-major, unswizzled core-matrix
+//     layout the tensor cores read (8 rows x 16 bytes per core matrix), one elected thread issues
+//     four tcgen05.mma (K = 16 each) into the tile's FP32 accumulator in tensor memory and commits
+//     them to an mbarrier, and after the last slice the four warps read the accumulator back
+//     (tcgen05.ld, one row per thread) and apply the epilogue.
 //
 // Every wait is bounded: an mbarrier wait that runs out sets an error flag (read with
 // st_b200_mlp_error) and the kernel drains and returns, freeing its tensor memory.
 #include <cstdint>
 #include <cstdio>
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -187,6 +190,29 @@ __device__ __forceinline__ void load_tile(unsigned char *dst, const __nv_bfloat1
     }
 }
 
+// one accumulator value of C (element `at`, column `col`) through the epilogue
+__device__ __forceinline__ void epilogue1(const GemmArgs &g, long long at, int col, float v) {
+    switch (g.epi) {
+        case EPI_BIAS_RELU_BF16:
+            static_cast<__nv_bfloat16 *>(g.C)[at] = __float2bfloat16_rn(fmaxf(v + g.bias[col], 0.f));
+            break;
+        case EPI_BIAS_F32:
+            static_cast<float *>(g.C)[at] = v + g.bias[col];
+            break;
+        case EPI_RELU_MASK_BF16:
+            static_cast<__nv_bfloat16 *>(g.C)[at] =
+                __bfloat162float(g.aux[at]) > 0.f ? __float2bfloat16_rn(v) : __float2bfloat16_rn(0.f);
+            break;
+        case EPI_F32:
+            static_cast<float *>(g.C)[at] = v;
+            break;
+        default:
+            atomicAdd(static_cast<float *>(g.C) + at, v);
+    }
+}
+
+// The product for operands TMA cannot address (neither stride 1, rows not 16 bytes apart or
+// unaligned bases): loads of any stride, one stage.
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_gemm(GemmArgs g) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -256,23 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_gemm(GemmArgs g) {
                 const int col = n0 + c0 + i;
                 if (col >= g.N) continue;
                 const long long at = row * g.ldc + col;
-                switch (g.epi) {
-                    case EPI_BIAS_RELU_BF16:
-                        static_cast<__nv_bfloat16 *>(g.C)[at] = __float2bfloat16_rn(fmaxf(v[i] + g.bias[col], 0.f));
-                        break;
-                    case EPI_BIAS_F32:
-                        static_cast<float *>(g.C)[at] = v[i] + g.bias[col];
-                        break;
-                    case EPI_RELU_MASK_BF16:
-                        static_cast<__nv_bfloat16 *>(g.C)[at] =
-                            __bfloat162float(g.aux[at]) > 0.f ? __float2bfloat16_rn(v[i]) : __float2bfloat16_rn(0.f);
-                        break;
-                    case EPI_F32:
-                        static_cast<float *>(g.C)[at] = v[i];
-                        break;
-                    default:
-                        atomicAdd(static_cast<float *>(g.C) + at, v[i]);
-                }
+                epilogue1(g, at, col, v[i]);
             }
         }
     }
@@ -281,6 +291,288 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_gemm(GemmArgs g) {
     if (!ok) mbar_wait(&bar, phase ^ 1u);  // a product still in flight finishes before its memory is freed
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(BN)));
+}
+
+// ---------------------------------------------------------------------------------------
+// The same product with both operands brought in by TMA
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// bounded wait that also gives up as soon as another role raised the abort flag
+__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, unsigned parity, volatile int *abort) {
+    const uint32_t a = smem_u32(bar);
+    for (unsigned it = 0; it < kSpinLimit; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (*abort) return false;
+    }
+    return false;
+}
+
+// one box of a tensor map -> this CTA's shared memory, its bytes counted on `bar`; x (the
+// contiguous dimension) is a multiple of 64 elements everywhere below
+__device__ __forceinline__ void tma_load(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// 32 bytes to global memory in one store (a whole sector per thread)
+__device__ __forceinline__ void store32(void *p, const uint32_t v[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+// Matrix descriptor of a 128-byte-swizzled tile as TMA leaves it (8 rows x 128 bytes per atom,
+// 1024 bytes).  K-major (a row holds 64 K values): row groups 1024 bytes apart.  MN-major (a row
+// holds 64 M or N values of one K): K groups 1024 bytes apart (stride offset), the next 64 M or N
+// values one 64-row box further (leading offset).
+constexpr uint32_t kBoxBytes = 64 * kBK * 2;  // an MN-major box: 64 values x 64 K
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr, bool mn_major) {
+    uint64_t d = uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) |
+                 (uint64_t(2) << 61);
+    return d | (uint64_t(mn_major ? (kBoxBytes >> 4) : 1u) << 16);
+}
+
+// Sixteen accumulator values of one row of C (columns col .. col + 15) through the epilogue
+__device__ __forceinline__ void epilogue16(const GemmArgs &g, long long row, int col, const float v[16], bool wide) {
+    const long long at = row * g.ldc + col;
+    if (wide && col + 16 <= g.N) {
+        if (g.epi == EPI_BIAS_RELU_BF16 || g.epi == EPI_RELU_MASK_BF16) {
+            float y[16];
+            if (g.epi == EPI_BIAS_RELU_BF16) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) y[i] = fmaxf(v[i] + __ldg(g.bias + col + i), 0.f);
+            } else {
+                const uint4 *a = reinterpret_cast<const uint4 *>(g.aux + at);
+                const uint4 a0 = a[0], a1 = a[1];
+                const uint32_t h[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    y[2 * i] = __uint_as_float(h[i] << 16) > 0.f ? v[2 * i] : 0.f;
+                    y[2 * i + 1] = __uint_as_float(h[i] & 0xffff0000u) > 0.f ? v[2 * i + 1] : 0.f;
+                }
+            }
+            uint32_t p[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                p[i] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(y[2 * i]))) |
+                       (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(y[2 * i + 1]))) << 16);
+            store32(static_cast<__nv_bfloat16 *>(g.C) + at, p);
+        } else if (g.epi == EPI_F32_ADD) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+                atomicAdd(reinterpret_cast<float4 *>(static_cast<float *>(g.C) + at + i),
+                          make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+        } else {
+            uint32_t p[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                p[i] = __float_as_uint(g.epi == EPI_BIAS_F32 ? v[i] + __ldg(g.bias + col + i) : v[i]);
+            store32(static_cast<float *>(g.C) + at, p);
+            store32(static_cast<float *>(g.C) + at + 8, p + 8);
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        if (col + i < g.N) epilogue1(g, at + i, col + i, v[i]);
+}
+
+// Operands whose rows TMA can address (one stride 1, the other a multiple of 8 values, 16-byte
+// aligned bases): persistent CTAs walk the (tile, K split) items; one thread keeps a ring of
+// A and B tiles filled with TMA loads, one issues the tensor-core products, eight warps run the
+// epilogue of the last item from one accumulator while the next item's products fill the
+// other.  Either operand may be stored with its M (N) index contiguous: its boxes hold 64 such
+// values by 64 K and the products read them transposed in place.  Rows and K beyond the
+// matrices arrive as zeros.
+// Against k_mlp_gemm (one stage, every wait exposed, element loads of transposed operands): the
+// sixteen 256-wide products of a gradient pass over 16,384 rows took 140 us each there and take
+// 17 here (bound by the traffic of their outputs and by filling a single wave of tiles); the
+// pass fell from 2.31 to 0.42 ms.
+constexpr int kPipeThreads = 320;             // warps 0-7 epilogue, 8 loader, 9 products
+constexpr int kPipeBytes = 192 * 1024;        // ring of operand tiles
+template <int BN>
+__global__ void __launch_bounds__(kPipeThreads, 1)
+    k_mlp_gemm_tma(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+                   const __grid_constant__ GemmArgs g, int tiles_m, int tiles_n, long long items, int a_mn, int b_mn) {
+    constexpr uint32_t kABytes = kBM * kBK * 2, kTile = kABytes + BN * kBK * 2;
+    constexpr int kStages = kPipeBytes / kTile;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = smem_raw + (1024u - (smem_u32(smem_raw) & 1023u)) % 1024u;
+    __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_free[2], drain;
+    __shared__ uint32_t tmem_sh;
+    __shared__ volatile int abort_flag;
+    __shared__ unsigned issued_sh, consumed_sh;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_free[i], 256);
+        }
+        mbar_init(&drain, 1);
+        abort_flag = 0;
+        issued_sh = consumed_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {  // two 128 x BN FP32 accumulators
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
+                     "r"(uint32_t(2 * BN)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_sh;
+    // item -> tile and K range [k0, k0 + kBK nk); an empty split has nk = 0
+    auto item = [&](long long it, int &m0, int &n0, int &k0, int &nk) {
+        m0 = int(it % tiles_m) * kBM;
+        n0 = int(it / tiles_m % tiles_n) * BN;
+        const long long kb = it / tiles_m / tiles_n * g.k_per_split;
+        const long long ke = min((long long)g.K, kb + g.k_per_split);
+        k0 = int(kb);
+        nk = ke > kb ? int((ke - kb + kBK - 1) / kBK) : 0;
+    };
+    int m0, n0, k0, nk;
+    if (warp == 8) {
+        // ---- loader ----
+        if (lane == 0) {
+            unsigned q = 0;
+            for (long long it = blockIdx.x; it < items && !abort_flag; it += gridDim.x) {
+                item(it, m0, n0, k0, nk);
+                for (int k = 0; k < nk; ++k, ++q) {
+                    const int slot = q % kStages, x = k0 + k * kBK;
+                    if (q >= kStages && !mbar_wait_or_abort(&empty[slot], ((q / kStages) - 1) & 1u, &abort_flag)) {
+                        abort_flag = 1;
+                        break;
+                    }
+                    unsigned char *sa = smem + slot * kTile, *sb = sa + kABytes;
+                    mbar_expect_tx(&full[slot], kTile);
+                    if (a_mn)
+                        for (int c = 0; c < kBM / 64; ++c) tma_load(sa + c * kBoxBytes, &ta, m0 + 64 * c, x, &full[slot]);
+                    else
+                        tma_load(sa, &ta, x, m0, &full[slot]);
+                    if (b_mn)
+                        for (int c = 0; c < BN / 64; ++c) tma_load(sb + c * kBoxBytes, &tb, n0 + 64 * c, x, &full[slot]);
+                    else
+                        tma_load(sb, &tb, x, n0, &full[slot]);
+                }
+            }
+            issued_sh = q;
+        }
+    } else if (warp == 9) {
+        // ---- products ----
+        if (lane == 0) {
+            const uint32_t idesc = instr_desc(BN) | (uint32_t(a_mn) << 15) | (uint32_t(b_mn) << 16);
+            // a K = 16 step: 32 bytes along a K-major row, two 8-K groups of an MN-major box
+            const uint32_t astep = a_mn ? 2048u : 32u, bstep = b_mn ? 2048u : 32u;
+            unsigned q = 0, u = 0;
+            bool ok = true;
+            for (long long it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                item(it, m0, n0, k0, nk);
+                if (nk == 0) continue;
+                const int b = u & 1;
+                if (u >= 2 && !mbar_wait_or_abort(&acc_free[b], ((u >> 1) - 1) & 1u, &abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int k = 0; k < nk; ++k, ++q) {
+                    const int slot = q % kStages;
+                    if (!mbar_wait_or_abort(&full[slot], (q / kStages) & 1u, &abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t sa = smem_u32(smem + slot * kTile), sb = sa + kABytes;
+#pragma unroll
+                    for (int j = 0; j < kBK / 16; ++j)
+                        mma_bf16(tmem + uint32_t(b * BN), sw128_desc(sa + j * astep, a_mn), sw128_desc(sb + j * bstep, b_mn),
+                                 idesc, (k > 0 || j > 0) ? 1u : 0u);
+                    mma_commit(&empty[slot]);
+                }
+                if (ok) mma_commit(&acc_full[b]);
+                ++u;
+            }
+            if (!ok) abort_flag = 1;
+            consumed_sh = q;
+            // every product this thread issued has finished before the CTA frees its memory
+            mma_commit(&drain);
+            mbar_wait(&drain, 0);
+        }
+    } else {
+        // ---- epilogue: warp w reads accumulator lanes 32 (w % 4) .. + 31 of half the columns ----
+        const int out_size = (g.epi == EPI_BIAS_RELU_BF16 || g.epi == EPI_RELU_MASK_BF16) ? 2 : 4;
+        // whole 32-byte stores (aux is shaped as C and read alongside)
+        const bool wide = ((reinterpret_cast<uintptr_t>(g.C) | uintptr_t(g.ldc * out_size)) & 31) == 0 &&
+                          (g.epi != EPI_RELU_MASK_BF16 || (reinterpret_cast<uintptr_t>(g.aux) & 15) == 0);
+        unsigned u = 0;
+        bool ok = true;
+        for (long long it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            item(it, m0, n0, k0, nk);
+            if (nk == 0) continue;
+            const int b = u & 1;
+            // warp-uniform: the tensor-memory loads below are warp-collective
+            if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&acc_full[b], (u >> 1) & 1u, &abort_flag))) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const long long row = m0 + (warp & 3) * 32 + lane;
+            constexpr int kHalf = BN / 2, kCols = kHalf < 64 ? kHalf : 64;
+            for (int c = (warp >> 2) * kHalf; c < (warp >> 2) * kHalf + kHalf; c += kCols) {
+                if (n0 + c >= g.N) break;
+                const uint32_t at = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(b * BN + c);
+                float v[kCols];
+                if (kCols == 64) {
+                    tmem_ld64(at, v);
+                } else {
+                    tmem_ld16(at, v);
+                    tmem_ld16(at + 16, v + 16);
+                }
+                if (row < g.M) {
+#pragma unroll
+                    for (int i = 0; i < kCols; i += 16) epilogue16(g, row, n0 + c + i, v + i, wide);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(&acc_free[b]);
+            ++u;
+        }
+        if (!ok) abort_flag = 1;
+    }
+    __syncthreads();
+    if (abort_flag) {
+        if (threadIdx.x == 0) {
+            atomicExch(g.err, 1u);
+            // operand copies issued but never consumed land before their shared memory goes away
+            for (unsigned q = consumed_sh; q < issued_sh; ++q) mbar_wait(&full[q % kStages], (q / kStages) & 1u);
+        }
+        __syncthreads();
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(2 * BN)));
 }
 
 // mean-squared-error loss over rows x cols outputs against float targets: dY = bf16(2 (y - t) /
@@ -426,38 +718,12 @@ struct FusedArgs {
     unsigned *err;
 };
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
 // one bulk copy global -> this CTA's shared memory, its bytes counted on `bar`
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
-}
-
-// bounded wait that also gives up as soon as another role raised the abort flag
-__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, unsigned parity, volatile int *abort) {
-    const uint32_t a = smem_u32(bar);
-    for (unsigned it = 0; it < kSpinLimit; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (*abort) return false;
-    }
-    return false;
 }
 
 // weight stages of one tile: the first layer's block, 4 per hidden layer, 4 per output chunk
@@ -781,6 +1047,77 @@ int launch_gemm(const GemmArgs &a, int splits, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }
 
+// The tensor map of one operand: `rows` x `k` values, element (r, j) at p[r lr + j lk].  K-major
+// (lk 1) boxes hold 64 K of `box_rows` rows, MN-major ones (lr 1) 64 rows of kBK K.  False when
+// TMA cannot address it.
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+bool operand_map(CUtensorMap &map, const __nv_bfloat16 *p, int rows, int k, long long lr, long long lk, int box_rows,
+                 int &mn_major) {
+    mn_major = lk != 1;
+    const long long ld = mn_major ? lk : lr;
+    if ((mn_major && lr != 1) || ld <= 0 || ld % 8 || ld >= (1ll << 38) || (reinterpret_cast<uintptr_t>(p) & 15))
+        return false;
+    const EncodeTiled encode = encode_tiled();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {cuuint64_t(mn_major ? rows : k), cuuint64_t(mn_major ? k : rows)};
+    const cuuint64_t stride[1] = {cuuint64_t(ld) * 2};
+    const cuuint32_t box[2] = {64u, cuuint32_t(mn_major ? kBK : box_rows)}, step[2] = {1u, 1u};
+    return encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16 *>(p), dims, stride, box, step,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// SMs of the current device, 0 on failure
+int device_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return n;
+}
+
+// 1 launched, -1 launch failure, 0: TMA cannot address the operands (the caller launches k_mlp_gemm)
+template <int BN>
+int launch_gemm_tma(const GemmArgs &a, int splits, cudaStream_t st) {
+    CUtensorMap ta, tb;
+    int a_mn = 0, b_mn = 0;
+    if (!operand_map(ta, a.A, a.M, a.K, a.lam, a.lak, kBM, a_mn) ||
+        !operand_map(tb, a.B, a.N, a.K, a.lbn, a.lbk, BN, b_mn))
+        return 0;
+    constexpr int smem = kPipeBytes + 1024;
+    // set on every call: the attribute belongs to the current device's context
+    if (cudaFuncSetAttribute(k_mlp_gemm_tma<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return -1;
+    const int sms = device_sms();
+    if (sms <= 0) return -1;
+    const long long tiles_m = (a.M + (long long)kBM - 1) / kBM, tiles_n = (a.N + (long long)BN - 1) / BN;
+    const long long items = tiles_m * tiles_n * splits;
+    k_mlp_gemm_tma<BN><<<unsigned(items < sms ? items : sms), kPipeThreads, smem, st>>>(
+        ta, tb, a, int(tiles_m), int(tiles_n), items, a_mn, b_mn);
+    return cudaGetLastError() == cudaSuccess ? 1 : -1;
+}
+
+// the TMA kernel where it can read the operands, else the one that reads any strides
+template <int BN>
+int launch_gemm_any(const GemmArgs &a, int splits, cudaStream_t st) {
+    const int rc = launch_gemm_tma<BN>(a, splits, st);
+    return rc != 0 ? rc : launch_gemm<BN>(a, splits, st);
+}
+
 // the fused kernel's shape rules; -1 or the packed size in bf16 elements
 long long packed_elems(int n_layers, const int *dims) {
     if (!dims || n_layers < 2 || n_layers > kMaxLayers) return -1;
@@ -844,9 +1181,9 @@ int st_b200_mlp_gemm(int m, int n, int k, const void *A, long long lam, long lon
     a.err = err_flag();
     if (!a.err) return -1;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (n >= 256) return launch_gemm<256>(a, splits, st);
-    if (n <= 64) return launch_gemm<64>(a, splits, st);
-    return launch_gemm<128>(a, splits, st);
+    if (n >= 256) return launch_gemm_any<256>(a, splits, st);
+    if (n <= 64) return launch_gemm_any<64>(a, splits, st);
+    return launch_gemm_any<128>(a, splits, st);
 }
 
 int st_b200_mlp_mse(int rows, int cols, const float *y, const float *target, long long ldt, void *dy, double *loss,

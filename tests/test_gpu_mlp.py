@@ -89,6 +89,26 @@ def test_gemm_matches_host(mlp_env, case):
     assert err <= tol, (err, tol)
 
 
+TMA_CASES = [  # as CASES; rows 16 bytes apart, which the TMA kernel takes, at the edges of its tiles
+    (1, 8, 8, False, False, 3, 1),             # one row, K below a tensor-core step
+    (128, 256, 16, False, False, 0, 1),        # the input layer's K
+    (129, 264, 72, False, False, 1, 1),        # one past every tile, N in the element epilogue's tail
+    (136, 64, 64, True, False, 3, 1),          # A's rows contiguous, B's K
+    (120, 72, 200, True, True, 3, 1),
+    (256, 520, 136, False, True, 0, 1),
+    (20_000, 512, 64, False, False, 2, 1),     # more tiles than SMs: both accumulators in turn
+    (264, 264, 4104, True, True, 4, 9),        # splits of 8 K blocks, the last one of a single K step
+    (256, 16, 640, True, True, 4, 7),          # 10 K blocks over 7 splits: empty ones at the end
+    (300, 130, 64, False, False, 4, 1),        # aligned operands, C's rows unaligned for wide stores
+]
+
+
+@pytest.mark.parametrize("case", TMA_CASES, ids=[f"{c[0]}x{c[1]}x{c[2]}-{int(c[3])}{int(c[4])}-e{c[5]}-s{c[6]}"
+                                                 for c in TMA_CASES])
+def test_gemm_tma_edges(mlp_env, case):
+    test_gemm_matches_host(mlp_env, case)
+
+
 @pytest.mark.parametrize("rows,cols,offset", [(1, 1, 0), (63, 7, 1), (512, 32, 0), (513, 33, 0), (2049, 256, 0),
                                               (1000, 1024, 3), (16384, 40, 0)])
 def test_colsum_matches_host(mlp_env, rows, cols, offset):
