@@ -126,6 +126,27 @@ def test_colsum_matches_host(mlp_env, rows, cols, offset):
     assert bool(((db.double() - want).abs() <= tol).all())
 
 
+@pytest.mark.parametrize("rows,cols,ldt,offset", [(1, 1, 1, 0), (1, 4, 4, 0), (3, 5, 5, 0), (37, 64, 80, 0),
+                                                  (129, 1024, 1024, 0), (129, 1024, 1024, 1), (4096, 1024, 1024, 0)])
+def test_mse_matches_host(mlp_env, rows, cols, ldt, offset):
+    """Loss and output gradient with contiguous, strided and unaligned targets: the gradient is the
+    bf16 rounding of the float expression, the loss a double sum (2^-53 per addition, of
+    non-negative terms)."""
+    torch, net = mlp_env
+    g = torch.Generator(device="cpu").manual_seed(rows * cols + offset)
+    y = torch.randn(rows, cols, generator=g).cuda()
+    t = torch.randn(rows * ldt + offset, generator=g).cuda()[offset:].view(rows, ldt)
+    dy = torch.empty(rows, cols, dtype=torch.bfloat16, device="cuda")
+    loss = torch.full((1,), 0.5, dtype=torch.float64, device="cuda")
+    assert net.api.lib.st_b200_mlp_mse(rows, cols, y.data_ptr(), t.data_ptr(), ldt, dy.data_ptr(), loss.data_ptr(),
+                                       net._s()) == 1
+    d = y - t[:, :cols]
+    scale = torch.tensor(2.0) / torch.tensor(float(rows * cols))
+    assert torch.equal(dy, (d * scale.cuda()).to(torch.bfloat16))
+    want = 0.5 + (d.double() ** 2).sum().item()
+    assert abs(loss.item() - want) <= 2.0 ** -53 * rows * cols * want + 1e-15
+
+
 def test_network_gradients_match_oracle(product):
     import torch
     import mlp_oracle
