@@ -237,7 +237,7 @@ def config_lines(api, args) -> dict:
         api.st_b200_set_records(ctx, 1 if records else 0)
         for m in maps:
             api.st_b200_add_flux_map(ctx, *m)
-        for w in range(3):  # warm-up: scene set-up, autotuning, buffers sized for the planned batches
+        for w in range(3):  # warm-up: scene set-up, buffers sized for the planned batches
             api.run(ctx, seed + 1000 + w)
         units = dev = wall = 0.0
         flux = None
@@ -523,7 +523,7 @@ def main():
     clk_summary = clk.summary()
     clk_mhz = clk_summary.get("sm_mhz") or 1965.0
     issue_peak = fm.issue_peak_per_s(clk_mhz)
-    group = {"k_probe": "probe group (k_sun_probe_exact or k_sun_candidates + k_sun_resolve, block-count scan, "
+    group = {"k_probe": "probe group (k_sun_probe_flat or k_sun_candidates + k_sun_resolve, block-count scan, "
                         "element sort)",
              "k_trace": "trace group (k_wf_first, k_wf_search, k_wf_shade, k_wf_finish)"}[dominant]
     roofline = {"bound": "fp64", "kernel": group, "achieved": ach, "peak": pk, "unit": "TFLOP/s",

@@ -87,7 +87,7 @@ typedef struct st_b200_stats {
     int gpu_launches;                     /* kernels launched by the run */
     unsigned long long h2d_bytes;         /* host -> device bytes copied by the run */
     unsigned long long d2h_bytes;         /* device -> host bytes copied by the run */
-    int probe_variant, trace_variant;     /* autotuned kernel variants used */
+    int probe_variant, trace_variant;     /* 0 (one variant of each kernel) */
     unsigned long long intersections;     /* records of the run by the reference's rules,
                                              counted on the device when records are off */
 } st_b200_stats;

@@ -953,6 +953,87 @@ void build_bvh(const std::vector<Elem> &els, std::vector<BvhNode> &nodes, std::v
     for (auto &it : its) items.push_back(it.j);
 }
 
+// Fixed-point scale of the sun-plane grid for the flat-rectangle probe (SunDev::fx_mul ...) and
+// the bound on its float test's error in a sun-plane coordinate.  A coordinate is U S cells from
+// the lower edge, U the uniform variate cut to 32 bits and S = extent / cell; the device
+// multiplies U by mul = floor(S 2^shift) and takes the cell from the product's high word and 23
+// bits of the place in the cell below it.  Error (m): the cut of U (extent 2^-32), of mul
+// (cell 2^-shift) and of the place (cell 2^-23); the float rounding of place, entry centre and
+// their difference (2.4e-7 of 1.5 cells and a disc radius); and the 1e-11 that the element test adds
+// to the direction's z component when it divides by it (element_test_flat), which moves the
+// hit 1.1e-11 of the ray's length per unit slope; half as much again for the rest.
+struct FlatProbe {
+    bool ok = false;
+    uint32_t mul[2] = {0, 0};
+    int shift[2] = {0, 0};
+    double eps = 0.0;
+};
+FlatProbe flat_probe_params(double W, double H, double cell, double rmax, const std::vector<Elem> &els,
+                            const double Rs[9]) {
+    FlatProbe f;
+    double zmax = 0.0;
+    for (const Elem &e : els) {
+        double p[3];
+        mulv(Rs, e.origin, p);
+        zmax = std::max(zmax, fabs(p[2]));
+    }
+    double cut = 0.0;
+    f.ok = true;
+    for (int q = 0; q < 2; ++q) {
+        const double ext = q ? H : W, S = ext / cell;
+        int b = 0;
+        while (b < 32 && ldexp(1.0, b) <= S) ++b;
+        f.shift[q] = std::min(22, 32 - b);
+        if (!(S > 0.0) || f.shift[q] < 9) f.ok = false;
+        f.mul[q] = f.ok ? uint32_t(floor(ldexp(S, f.shift[q]))) : 0;
+        if (f.mul[q] == 0) f.ok = false;
+        cut = std::max(cut, ldexp(ext, -32) + cell * (ldexp(1.0, -f.shift[q]) + ldexp(1.0, -23)));
+    }
+    f.eps = 1.5 * (cut + 2.4e-7 * (1.5 * cell + rmax) + 1.1e-11 * (1.0e4 + zmax + rmax));
+    return f;
+}
+
+// Occupancy bitmap over the sun-plane box (SunDev::occ): the finest power-of-two division of the
+// grid's cells that fits kMaxOccWords, a bit set where a footprint, widened by the probe's error
+// bound, may reach into its square.
+struct OccupancyMap {
+    int k = 0, nx = 0, ny = 0, stride = 0;
+    double side = 0.0, pad = 0.0;
+    std::vector<uint32_t> bits;
+    void size(int cx, int cy, double cell, const FlatProbe &fp) {
+        auto count = [](int n, int kk) { return kk >= 0 ? n << kk : (n + (1 << -kk) - 1) >> -kk; };
+        for (k = 2;; --k) {
+            nx = count(cx, k);
+            ny = count(cy, k);
+            stride = (nx + 31) / 32;
+            if (size_t(stride) * size_t(ny) <= size_t(kMaxOccWords) || k <= -9) break;
+        }
+        bits.assign(size_t(stride) * size_t(ny), 0u);
+        side = ldexp(cell, -k);
+        pad = 4.0 * fp.eps;
+    }
+    template <typename F>
+    void visit(double x, double y, double hx, double hy, F inside) {
+        const int x0 = std::max(0, int(floor((x - hx) / side))), x1 = std::min(nx - 1, int(floor((x + hx) / side)));
+        const int y0 = std::max(0, int(floor((y - hy) / side))), y1 = std::min(ny - 1, int(floor((y + hy) / side)));
+        for (int iy = y0; iy <= y1; ++iy)
+            for (int ix = x0; ix <= x1; ++ix)
+                if (inside((ix + 0.5) * side - x, (iy + 0.5) * side - y))
+                    bits[size_t(iy) * size_t(stride) + size_t(ix >> 5)] |= 1u << (ix & 31);
+    }
+    // parallelogram about (x, y) of half extents (hx, hy) with dual basis rows (i[0], i[1]), (i[2], i[3])
+    void mark(double x, double y, double hx, double hy, const double i[4]) {
+        const double h = 0.5 * side + pad;  // half a square, widened
+        const double lu = 1.0 + 1e-5 + (fabs(i[0]) + fabs(i[1])) * h, lv = 1.0 + 1e-5 + (fabs(i[2]) + fabs(i[3])) * h;
+        visit(x, y, hx * (1.0 + 1e-5) + pad, hy * (1.0 + 1e-5) + pad, [&](double qx, double qy) {
+            return fabs(i[0] * qx + i[1] * qy) <= lu && fabs(i[2] * qx + i[3] * qy) <= lv;
+        });
+    }
+    void mark_disc(double x, double y, double r) {
+        visit(x, y, r + pad, r + pad, [](double, double) { return true; });
+    }
+};
+
 // ---------------- the sun frame and sun box (suntoprimarystage.cpp:59-293) ----------------
 bool sun_setup(Context *cx, HostScene &hs) {
     StageM &st = cx->stages[0];
@@ -1094,6 +1175,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
     hs.cell_xa.clear();
     hs.cell_xb.clear();
     hs.cell_xc.clear();
+    hs.occ.clear();
     if (!sun.point_source && st.elems.size() >= 4) {
         bool bounded = true;
         double rmax = 0;
@@ -1117,23 +1199,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
             // keep the grid within the context's cell budget (~4M cells for a single run)
             while ((W / cell + 1) * (H / cell + 1) > cx->sun_grid_cells) cell *= 1.5;
             const int nx = std::max(1, int(ceil(W / cell))), ny = std::max(1, int(ceil(H / cell)));
-            std::vector<std::vector<int>> cells(size_t(nx) * ny);
-            for (size_t j = 0; j < st.elems.size(); ++j) {
-                const double pad = rad[j] * (1.0 + 1e-9) + 1e-6 * (1.0 + fabs(cx_[j]) + fabs(cy_[j]));
-                const int x0 = std::max(0, int(floor((cx_[j] - pad - sun.xmin) / cell)));
-                const int x1 = std::min(nx - 1, int(floor((cx_[j] + pad - sun.xmin) / cell)));
-                const int y0 = std::max(0, int(floor((cy_[j] - pad - sun.ymin) / cell)));
-                const int y1 = std::min(ny - 1, int(floor((cy_[j] + pad - sun.ymin) / cell)));
-                for (int gy = y0; gy <= y1; ++gy)
-                    for (int gx = x0; gx <= x1; ++gx) {
-                        // distance from the disc centre to the cell rectangle
-                        const double ax = sun.xmin + gx * cell, bx = ax + cell;
-                        const double ay = sun.ymin + gy * cell, by = ay + cell;
-                        const double ddx = std::max(std::max(ax - cx_[j], 0.0), cx_[j] - bx);
-                        const double ddy = std::max(std::max(ay - cy_[j], 0.0), cy_[j] - by);
-                        if (ddx * ddx + ddy * ddy <= pad * pad) cells[size_t(gy) * nx + gx].push_back(int(j));
-                    }
-            }
+            const FlatProbe fp = flat_probe_params(W, H, cell, rmax, st.elems, Rs);
             // Per element a float disc (centre, radius) and a parallelogram about the same
             // centre for the probe's pre-tests; both contain every sun-plane point whose ray can
             // be accepted by the element.
@@ -1193,17 +1259,49 @@ bool sun_setup(Context *cx, HostScene &hs) {
                 memcpy(&w, &bits, 4);
                 disc[j] = float4{float(ccx), float(ccy), float(fr), w};
             }
-            // Exact footprints for first stages of flat rectangles (the mixed-precision probe
+            // Cells: an element is listed where both its disc and its parallelogram reach (the second
+            // leaves a third of the disc's cells on a heliostat field); elements that accept no hit
+            // (disabled, or flat beyond their ZAperture, element_test_flat) are listed nowhere.
+            bool exact = fp.ok;
+            for (const Elem &e : st.elems)
+                if (e.stype != 3 || char(tolower(e.shape)) != 'r') exact = false;
+            auto never = [&](const Elem &e) { return !e.enabled || (exact && !(0.0 <= e.zap)); };
+            std::vector<std::vector<int>> cells(size_t(nx) * ny);
+            for (size_t j = 0; j < st.elems.size(); ++j) {
+                if (never(st.elems[j])) continue;
+                const double pad = rad[j] * (1.0 + 1e-9) + 1e-6 * (1.0 + fabs(cx_[j]) + fabs(cy_[j])) + 2.0 * fp.eps;
+                const int x0 = std::max(0, int(floor((cx_[j] - pad - sun.xmin) / cell)));
+                const int x1 = std::min(nx - 1, int(floor((cx_[j] + pad - sun.xmin) / cell)));
+                const int y0 = std::max(0, int(floor((cy_[j] - pad - sun.ymin) / cell)));
+                const int y1 = std::min(ny - 1, int(floor((cy_[j] + pad - sun.ymin) / cell)));
+                for (int gy = y0; gy <= y1; ++gy)
+                    for (int gx = x0; gx <= x1; ++gx) {
+                        // distance from the disc centre to the cell rectangle
+                        const double ax = sun.xmin + gx * cell, bx = ax + cell;
+                        const double ay = sun.ymin + gy * cell, by = ay + cell;
+                        const double ddx = std::max(std::max(ax - cx_[j], 0.0), cx_[j] - bx);
+                        const double ddy = std::max(std::max(ay - cy_[j], 0.0), cy_[j] - by);
+                        if (ddx * ddx + ddy * ddy > pad * pad) continue;
+                        // the parallelogram's rows at the cell's centre, widened by half a cell
+                        const double qx = 0.5 * (ax + bx) - disc[j].x, qy = 0.5 * (ay + by) - disc[j].y;
+                        const double h = 0.5 * cell + 2.0 * fp.eps + 4e-7 * (fabs(qx) + fabs(qy) + box_ext);
+                        const float4 r = par[j];
+                        if (fabs(r.x * qx + r.y * qy) <= 1.0 + 1e-5 + (fabs(r.x) + fabs(r.y)) * h &&
+                            fabs(r.z * qx + r.w * qy) <= 1.0 + 1e-5 + (fabs(r.z) + fabs(r.w)) * h)
+                            cells[size_t(gy) * nx + gx].push_back(int(j));
+                    }
+            }
+            // Exact footprints for first stages of flat rectangles (k_sun_probe_flat
             // decides hit and nearest element in float and defers to double within its
             // rounding margins): a sun-frame ray (x, y) meets the plane of element j at depth
             // z0 + gx qx + gy qy, q = (x, y) - centre, inside the rectangle when
             // |i00 qx + i01 qy| <= 1 and |i10 qx + i11 qy| <= 1 (the rectangle's half-axes
             // projected along the sun's z, inverted).  Coordinates are taken relative to the
             // lower corner of the entry's cell, so that floats hold them to ~1e-6 m.
-            bool exact = true;
-            for (const Elem &e : st.elems)
-                if (e.stype != 3 || char(tolower(e.shape)) != 'r') exact = false;
+            OccupancyMap occ;
+            if (exact) occ.size(nx, ny, cell, fp);
             std::vector<float4> xb(exact ? st.elems.size() : 0), xc(exact ? st.elems.size() : 0);
+            std::vector<float> xtol(exact ? st.elems.size() : 0, 0.f);
             std::vector<double> ecx(exact ? st.elems.size() : 0), ecy(exact ? st.elems.size() : 0);
             if (exact) {
                 for (size_t j = 0; j < st.elems.size(); ++j) {
@@ -1223,14 +1321,22 @@ bool sun_setup(Context *cx, HostScene &hs) {
                     ecx[j] = c2[0];
                     ecy[j] = c2[1];
                     xb[j] = float4{0.f, 0.f, 0.f, 0.f};
-                    if (!e.enabled || !(0.0 <= e.zap)) {
-                        xc[j] = float4{0.f, 0.f, INFINITY, 0.f};  // never accepted (element_test_flat)
-                    } else if (!(fabs(det) > 1e-3 * la * lb) || !(fabs(n2[2]) > 1e-3)) {
-                        xc[j] = float4{0.f, 0.f, NAN, 0.f};  // near edge-on: always decided in double
+                    if (never(e)) continue;
+                    if (!(fabs(det) > 1e-3 * la * lb) || !(fabs(n2[2]) > 1e-3)) {
+                        xc[j] = float4{0.f, 0.f, 0.f, INFINITY};  // near edge-on: always decided in double
+                        occ.mark_disc(c2[0] - sun.xmin, c2[1] - sun.ymin, disc[j].z + 2.0 * fp.eps);
                     } else {
-                        xb[j] = float4{float(b2[1] / det), float(-b2[0] / det), float(-a2[1] / det),
-                                       float(a2[0] / det)};
-                        xc[j] = float4{float(-n2[0] / n2[2]), float(-n2[1] / n2[2]), float(c2[2]), 0.f};
+                        const double i4[4] = {b2[1] / det, -b2[0] / det, -a2[1] / det, a2[0] / det};
+                        const double gx = -n2[0] / n2[2], gy = -n2[1] / n2[2];
+                        // margins over the cells the element is listed in, |q| <= Q there: the float
+                        // rounding of (u, v) and of the depth, and the coordinates' own error
+                        const double Q = disc[j].z + 1.5 * cell, err = fp.eps * (1.0 + fabs(gx) + fabs(gy));
+                        const double row = std::max(fabs(i4[0]) + fabs(i4[1]), fabs(i4[2]) + fabs(i4[3]));
+                        xb[j] = float4{float(i4[0]), float(i4[1]), float(i4[2]), float(i4[3])};
+                        xc[j] = float4{float(gx), float(gy), float(c2[2]), float((6e-7 * Q + err) * row + 1e-6)};
+                        xtol[j] = float(1e-6 * (fabs(c2[2]) + (fabs(gx) + fabs(gy)) * Q) + err + 1e-5);
+                        occ.mark(c2[0] - sun.xmin, c2[1] - sun.ymin, fabs(a2[0]) + fabs(b2[0]),
+                                 fabs(a2[1]) + fabs(b2[1]), i4);
                     }
                 }
             }
@@ -1245,8 +1351,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
                     hs.cell_disc.push_back(disc[j]);
                     hs.cell_par.push_back(par[j]);
                     if (exact) {
-                        const float r = disc[j].z;
-                        hs.cell_xa.push_back(float4{float(ecx[j] - x0c), float(ecy[j] - y0c), r * r, disc[j].w});
+                        hs.cell_xa.push_back(float4{float(ecx[j] - x0c), float(ecy[j] - y0c), xtol[j], disc[j].w});
                         hs.cell_xb.push_back(xb[j]);
                         hs.cell_xc.push_back(xc[j]);
                     }
@@ -1255,6 +1360,18 @@ bool sun_setup(Context *cx, HostScene &hs) {
                 hs.cell_start[2 * c + 1] = at;
             }
             sd.exact_flat = exact ? 1 : 0;
+            if (exact) {
+                sd.fx_mul = fp.mul[0];
+                sd.fy_mul = fp.mul[1];
+                sd.fx_shift = fp.shift[0];
+                sd.fy_shift = fp.shift[1];
+                sd.fcell = float(cell);
+                sd.occ_shx = fp.shift[0] - occ.k;
+                sd.occ_shy = fp.shift[1] - occ.k;
+                sd.occ_stride = occ.stride;
+                sd.occ_words = int(occ.bits.size());
+                hs.occ.swap(occ.bits);
+            }
             sd.grid_on = 1;
             sd.gnx = nx;
             sd.gny = ny;
@@ -1739,6 +1856,7 @@ bool build_position(const Context *cx, const HostScene &hs, const double sun_xyz
     out.cell_xa.swap(h.cell_xa);
     out.cell_xb.swap(h.cell_xb);
     out.cell_xc.swap(h.cell_xc);
+    out.occ.swap(h.occ);
     if (target) {
         const StageRec &sr = hs.dev.stages[0];
         out.rot.resize(size_t(sr.n_elem) * 9);

@@ -29,6 +29,7 @@ struct HostScene {
     std::vector<float4> cell_disc;  // sun-plane grid entries: disc centre x, y, radius, element
     std::vector<float4> cell_par;   // sun-plane grid entries: footprint parallelogram (dual basis rows)
     std::vector<float4> cell_xa, cell_xb, cell_xc;  // sun-plane grid entries: exact flat footprints (SunDev)
+    std::vector<uint32_t> occ;  // occupancy bitmap of the exact flat footprints (SunDev)
     std::vector<double> inv_cdf;  // table-sunshape inverse CDF (kSunInvCells + 1 entries)
     SceneDev dev;  // stages, sun scalars and flags; device pointers are filled by gpu_run
 };
@@ -100,6 +101,7 @@ struct SunPosition {
     SunDev sun;                       // device pointers are filled by gpu_run_batch
     std::vector<int> cell_start;
     std::vector<float4> cell_disc, cell_par, cell_xa, cell_xb, cell_xc;
+    std::vector<uint32_t> occ;
     std::vector<double> rot;          // tracking: the first stage's re-aimed rotations, 9 per element
                                       // (empty: the scene's elements as they are)
     uint64_t n_hits = 0;

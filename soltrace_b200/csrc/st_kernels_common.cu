@@ -12,6 +12,29 @@ void launch_sun_candidates(const SceneDev &S, uint64_t s0, uint32_t n, const Pro
     cudaMemsetAsync(o.cand_count, 0, sizeof(uint32_t), st);
     k_sun_candidates<<<nblocks, kProbeBlock, 0, st>>>(S, s0, n, o, rs);
 }
+bool launch_sun_probe_flat(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
+                           cudaStream_t st) {
+    // outputs a caller without room for the undecided rays (or with one word per ray) asks for
+    // come from the general grid probe
+    if (!S.sun.exact_flat || !S.stages[0].flat_only || !o.amb || !o.cand_el || !o.hit_mask || o.hit_elem) return false;
+    const int smem = kFlatBlock / 32 * kFlatWarpBytes + S.sun.occ_words * int(sizeof(uint32_t));
+    if (cudaFuncSetAttribute(k_sun_probe_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return false;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaMemsetAsync(o.cand_count, 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(o.amb_count, 0, sizeof(uint32_t), st);
+    FlatKeys keys;
+    for (uint32_t r = 0; r < 7; ++r) {
+        keys.k0[r] = S.seed + (r + 3) * 0x9E3779B9u;
+        keys.k1[r] = 0x50C7A5E1u + (r + 3) * 0xBB67AE85u;
+    }
+    // persistent grid; fewer blocks where each warp would get less than one unit of kProbeBlock rays
+    const uint32_t blocks = std::max(1u, (n + kFlatBlock * 8 - 1) / (kFlatBlock * 8));
+    k_sun_probe_flat<<<std::min<uint32_t>(blocks, uint32_t(2 * sms)), kFlatBlock, smem, st>>>(S, keys, s0, n, o, rs);
+    return true;
+}
 void launch_offsets(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, cudaStream_t st) {
     k_offsets<<<1, 1024, 0, st>>>(counts, nb, offsets, total);
 }

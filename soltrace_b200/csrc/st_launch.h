@@ -12,10 +12,19 @@ constexpr int kResolveBlock = 128;  // threads per block of the grid probe's ele
 constexpr int kCandPerThread = 8;   // sun rays per thread of the grid probe's pre-test kernel
 constexpr int kCandRays = kProbeBlock * kCandPerThread;
 constexpr int kTraceBlock = 128;
-// register-budget variants of the probe and trace kernels (minimum resident blocks per
-// SM given to __launch_bounds__); all compute the same results
-constexpr int kProbeVariants = 3;
-constexpr int kProbeMinBlocks[kProbeVariants] = {4, 6, 8};
+// Probe of flat rectangles (k_sun_probe_flat): 24 warps a block, two blocks a SM (42 registers a
+// thread; 109 KB of shared memory a block with the largest occupancy bitmap)
+constexpr int kFlatBlock = 768;
+constexpr int kFlatSeg = 1024;      // sun rays of a warp's segment (32 mask words)
+constexpr int kFlatQueue = 96;      // rays a warp queues for the footprint test (31 + 64, one spare)
+constexpr int kFlatHits = 96;       // hits a warp gathers before listing them
+constexpr int kFlatWarpBytes = kFlatQueue * (8 + 2) + kFlatHits * 8 + kFlatSeg / 8;
+struct FlatKeys {                   // Philox keys of rounds 4 to 10
+    uint32_t k0[7], k1[7];
+};
+// resident blocks per SM asked of the grid probe's element-test kernel (register budget): on the
+// 2,000-heliostat field 2^24 sun rays took 147 us at 6, 142 at 8 and 150 at 4
+constexpr int kResolveMinBlocks = 6;
 // resident blocks per SM asked of the trace's shade and search kernels (register budget)
 constexpr int kWfShadeMinBlocks = 4;
 constexpr int kWfSearchMinBlocks = 4;
@@ -41,10 +50,6 @@ constexpr int kWfFirstFlatMinBlocksMixed = ST_FIRST_FLAT_MINB_MIXED;  // the sam
 // than 4 and no slower than 6) and mixed precision (4; 5 and 6 no faster)
 constexpr int kWfClosedShadeMinBlocks = 5;
 constexpr int kWfClosedShadeMinBlocksMixed = 4;
-#ifndef ST_EXACT_PROBE_MINB
-#define ST_EXACT_PROBE_MINB 8
-#endif
-constexpr int kExactProbeMinBlocks = ST_EXACT_PROBE_MINB;  // mixed probe of flat rectangles (k_sun_probe_exact)
 
 enum RunFlags : unsigned {
     kFlagHitCap = 1u,         // a ray reached kMaxHitsPerStage in one stage
@@ -132,7 +137,7 @@ struct ReplayIn {
 //                 probe's candidates, or (with cand_el) every ray of the other probes;
 //   cand_el       optional: element + 1 or 0 per list entry;
 //   hit_mask      optional: one bit per ray, set for a hit (hit_mask_words(n) words);
-//   amb, amb_count  room for n ray indices and their count (k_sun_probe_exact only).
+//   amb, amb_count  room for n ray indices and their count (k_sun_probe_flat only).
 // One numbered hit of a batch, sorted by first-stage element: its sun-ray index, the element
 // and its rank among the batch's hits in sun-ray order (its ray number less the batch's base);
 // one 16-byte store per hit when the sort scatters it.
@@ -146,21 +151,23 @@ struct ProbeOut {
     uint32_t *hit_elem;
     uint32_t *cand, *cand_count, *cand_el;
     uint32_t *hit_mask;
-    uint32_t *amb, *amb_count;  // mixed probe of flat rectangles: rays left to the double search
+    uint32_t *amb, *amb_count;  // probe of flat rectangles: rays left to the double search
 };
-// hit-mask words for n sun rays, rounded up to whole blocks of the widest probe variant
-// (16 rays per thread): every probe kernel writes the words of its blocks in full
-constexpr int kMaskRays = kProbeBlock * 16;
+// hit-mask words for n sun rays, rounded up to whole blocks of the pre-test kernel, the widest:
+// every probe kernel writes the words of its blocks in full
+constexpr int kMaskRays = kCandRays;
 constexpr size_t hit_mask_words(uint64_t n) { return size_t((n + kMaskRays - 1) / kMaskRays) * (kMaskRays / 32); }
-// rays per thread of the mixed flat-rectangle probe, per autotuner variant
-constexpr int kExactRpt[kProbeVariants] = {4, 8, 16};
 
 // First-stage probe of sun rays [s0, s0 + n) into `o`.  Returns the number of kernels
 // launched.
 int launch_probe_fp64(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
-                      int variant, cudaStream_t st);
+                      cudaStream_t st);
 int launch_probe_mixed(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
-                       int variant, cudaStream_t st);
+                       cudaStream_t st);
+// flat-rectangle first stages, both precisions: true when the scene and the outputs `o` take
+// k_sun_probe_flat (launched; the undecided rays in o.amb are left to k_sun_resolve_amb)
+bool launch_sun_probe_flat(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
+                           cudaStream_t st);
 // first kernel of the grid probe (shared by both precisions)
 void launch_sun_candidates(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
                            cudaStream_t st);

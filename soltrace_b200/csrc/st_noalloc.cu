@@ -170,7 +170,7 @@ extern "C" int st_b200_probe_noalloc(st_context_t pcxt, unsigned int seed, unsig
     S.sun.cell_start = d_cells;
     S.sun.cell_disc = d_cdisc;
     S.sun.cell_par = d_cpar;
-    S.sun.exact_flat = 0;  // FP64 probe: the exact flat footprints are not carved out
+    S.sun.exact_flat = 0;  // the exact flat footprints are not carved out: the general grid probe
     S.sun.inv_cdf = nullptr;
     S.optics = nullptr;
     S.tables = nullptr;
@@ -198,7 +198,7 @@ extern "C" int st_b200_probe_noalloc(st_context_t pcxt, unsigned int seed, unsig
     po.hit_elem = d_hit_elem;
     po.cand = d_cand + 1;
     po.cand_count = d_cand;
-    launch_probe_fp64(S, s0, n, po, d_rs, 0, st);
+    launch_probe_fp64(S, s0, n, po, d_rs, st);
     launch_offsets(d_counts, nb, d_offsets, d_total, st);
     launch_compact(s0, n, d_hit_elem, d_counts, d_offsets, reinterpret_cast<uint64_t *>(hit_sid), hit_elem, st);
     uint32_t total = 0;

@@ -106,15 +106,9 @@ struct Workspace {
     size_t rec_host_bytes = 0;
     bool rec_host_pinned = false;
     // batched runs: per-position sun tables, element copies, run states, counters, accumulators
-    DevBuf pos_cells, pos_disc, pos_par, pos_xa, pos_xb, pos_xc, pos_elems, pos_rot, pos_rs, pos_ctr, pos_acc;
-    DevBuf cell_xa, cell_xb, cell_xc;  // exact flat footprints of the sun-plane grid
+    DevBuf pos_cells, pos_disc, pos_par, pos_xa, pos_xb, pos_xc, pos_occ, pos_elems, pos_rot, pos_rs, pos_ctr, pos_acc;
+    DevBuf cell_xa, cell_xb, cell_xc, occ;  // exact flat footprints of the sun-plane grid
     std::vector<cudaEvent_t> events;
-    // autotuned kernel variants per precision (FP64, mixed), chosen on the first run
-    struct Tuning {
-        bool done = false;
-        int probe = 0;
-    } tune[2];
-    DevBuf tune_rs;
     ~Workspace() {
         if (device >= 0) cudaSetDevice(device);
         for (int k = 0; k < 2; ++k)
@@ -156,58 +150,6 @@ static cudaError_t probe_buffers(Workspace &ws, uint64_t n, ProbeOut &o) {
     o.cand_el = ws.cand_el.as<uint32_t>();
     o.hit_mask = ws.hit_mask.as<uint32_t>();
     return cudaSuccess;
-}
-
-// Autotuner: time every variant of the probe (register budgets, or rays per thread of the
-// mixed flat-rectangle probe) on the same 2^24 sun rays (indices 0.., outputs discarded into
-// scratch buffers: enough blocks to fill the GPU at every variant's rays per block, as the
-// 2^26-ray batches do) and keep the fastest for this workspace and precision.  Variants share
-// their arithmetic, so the choice changes timing only.
-static cudaError_t autotune(Workspace &ws, const SceneDev &S0, int precision, uint64_t max_sun, cudaStream_t st,
-                            int &launches) {
-    Workspace::Tuning &tu = ws.tune[precision ? 1 : 0];
-    const uint64_t n = std::min<uint64_t>(uint64_t(1) << 24, max_sun);
-    if (n == 0) return cudaSuccess;
-    cudaError_t e;
-    ProbeOut po;
-    if ((e = probe_buffers(ws, n, po)) || (e = ws.tune_rs.ensure(sizeof(RunState)))) return e;
-    SceneDev S = S0;
-    S.n_flux = 0;
-    RunState r0;
-    memset(&r0, 0, sizeof r0);
-    r0.target = ~0ull;
-    RunState *rs = ws.tune_rs.as<RunState>();
-    cudaMemcpyAsync(rs, &r0, sizeof r0, cudaMemcpyHostToDevice, st);
-    cudaEvent_t ev[2 * kProbeVariants];
-    for (auto &x : ev) cudaEventCreate(&x);
-    auto probe = [&](int v) {
-        if (precision)
-            launches += launch_probe_mixed(S, 0, uint32_t(n), po, rs, v, st);
-        else
-            launches += launch_probe_fp64(S, 0, uint32_t(n), po, rs, v, st);
-    };
-    probe(0);  // warm the caches
-    for (int v = 0; v < kProbeVariants; ++v) {
-        cudaEventRecord(ev[2 * v], st);
-        probe(v);
-        cudaEventRecord(ev[2 * v + 1], st);
-    }
-    e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) {
-        float best = 1e30f;
-        for (int v = 0; v < kProbeVariants; ++v) {
-            float ms = 0;
-            cudaEventElapsedTime(&ms, ev[2 * v], ev[2 * v + 1]);
-            if (ms < best * 0.98f) {
-                best = ms;
-                tu.probe = v;
-            }
-        }
-        tu.done = true;
-    }
-    for (auto &x : ev) cudaEventDestroy(x);
-    return e;
 }
 
 // trace state and queues for up to `cap` rays: one search queue per search kind among the
@@ -471,6 +413,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     CK(upload(ws.cell_xa, hs.cell_xa, st, out.h2d_bytes));
     CK(upload(ws.cell_xb, hs.cell_xb, st, out.h2d_bytes));
     CK(upload(ws.cell_xc, hs.cell_xc, st, out.h2d_bytes));
+    CK(upload(ws.occ, hs.occ, st, out.h2d_bytes));
     CK(upload(d_inv_cdf, hs.inv_cdf, st, out.h2d_bytes));
     CK(upload(d_expos, rq.ex_pos, st, out.h2d_bytes));
     CK(upload(d_excos, rq.ex_cos, st, out.h2d_bytes));
@@ -495,6 +438,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     S.sun.cell_xa = ws.cell_xa.as<float4>();
     S.sun.cell_xb = ws.cell_xb.as<float4>();
     S.sun.cell_xc = ws.cell_xc.as<float4>();
+    S.sun.occ = ws.occ.as<uint32_t>();
     if (hs.cell_xa.size() != hs.cell_disc.size() || hs.cell_xa.empty()) S.sun.exact_flat = 0;
     S.sun.inv_cdf = hs.inv_cdf.empty() ? nullptr : d_inv_cdf.as<double>();
     S.seed = rq.seed;
@@ -551,10 +495,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     CK(d_ecursor.ensure(size_t(n_elem0) * 4));
     CK(d_etotal.ensure(8));
     unsigned long long rec_cap = 0, save_cap = 0;
-    Workspace::Tuning &tu = ws.tune[rq.precision ? 1 : 0];
-    if (!tu.done && !explicit_mode && !rq.replay) CK(autotune(ws, S, rq.precision, rq.max_sun, st, out.gpu_launches));
-    out.probe_variant = tu.probe;
-    out.trace_variant = 0;
     (void)dev_sms;
     CK(cudaStreamSynchronize(st));
     out.setup_ms = ms_since(t_setup);
@@ -787,9 +727,9 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 CK(cudaEventRecord(p0, st));
                 if (n > 0) {
                     if (rq.precision)
-                        out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs, tu.probe, st);
+                        out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs, st);
                     else
-                        out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs, tu.probe, st);
+                        out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs, st);
                     launch_scan(po.block_counts, nb, d_offsets.as<uint32_t>(), d_total.as<uint32_t>(),
                                 ws.scan_parts.as<uint32_t>(), st);
                     out.gpu_launches += 2;
@@ -1053,12 +993,12 @@ namespace {
 // Where a chunk's positions sit in the device tables (and in a staging area laid out the
 // same way: one region per array, positions end to end).
 struct PosLayout {
-    std::vector<size_t> off_cells, off_disc, off_rot;
-    size_t n_cells = 0, n_disc = 0, n_rot = 0;
+    std::vector<size_t> off_cells, off_disc, off_rot, off_occ;
+    size_t n_cells = 0, n_disc = 0, n_rot = 0, n_occ = 0;
     bool all_exact = true;
-    size_t b_cells = 0, b_disc = 0, b_rot = 0, nx = 0, b_all = 0;
+    size_t b_cells = 0, b_disc = 0, b_rot = 0, b_occ = 0, nx = 0, b_all = 0;
     explicit PosLayout(const std::vector<SunPosition> &pos) : off_cells(pos.size()), off_disc(pos.size()),
-                                                              off_rot(pos.size()) {
+                                                              off_rot(pos.size()), off_occ(pos.size()) {
         for (const SunPosition &sp : pos)
             if (!sp.sun.exact_flat || sp.cell_xa.size() != sp.cell_disc.size() || sp.cell_xa.empty()) all_exact = false;
         for (size_t p = 0; p < pos.size(); ++p) {
@@ -1068,15 +1008,18 @@ struct PosLayout {
             n_disc += pos[p].cell_disc.size();
             off_rot[p] = n_rot;
             n_rot += pos[p].rot.size();
+            off_occ[p] = n_occ;
+            n_occ += pos[p].occ.size();
         }
         nx = all_exact ? 3 : 0;
         b_cells = n_cells * sizeof(int);
         b_disc = n_disc * sizeof(float4);
         b_rot = n_rot * sizeof(double);
-        b_all = b_cells + (2 + nx) * b_disc + b_rot;
+        b_occ = n_occ * sizeof(uint32_t);
+        b_all = b_cells + (2 + nx) * b_disc + b_rot + b_occ;
     }
-    // region starts in a staging area: cells, disc, par, xa, xb, xc, rot
-    void regions(char *base, char *r[7]) const {
+    // region starts in a staging area: cells, disc, par, xa, xb, xc, rot, occ
+    void regions(char *base, char *r[8]) const {
         r[0] = base;
         r[1] = r[0] + b_cells;
         r[2] = r[1] + b_disc;
@@ -1084,6 +1027,7 @@ struct PosLayout {
         r[4] = r[3] + (nx ? b_disc : 0);
         r[5] = r[4] + (nx ? b_disc : 0);
         r[6] = r[5] + (nx ? b_disc : 0);
+        r[7] = r[6] + b_rot;
     }
 };
 }  // namespace
@@ -1122,7 +1066,7 @@ bool stage_positions(Workspace &ws, int slot, const std::vector<SunPosition> &po
         }
         ws.pos_host_bytes[slot] = want;
     }
-    char *r[7];
+    char *r[8];
     L.regions(static_cast<char *>(ws.pos_host[slot]), r);
     auto cp = [](char *dst, const void *src, size_t bytes) {
         if (bytes) memcpy(dst, src, bytes);
@@ -1139,6 +1083,7 @@ bool stage_positions(Workspace &ws, int slot, const std::vector<SunPosition> &po
             cp(r[5] + od, sp.cell_xc.data(), nd);
         }
         cp(r[6] + L.off_rot[p] * sizeof(double), sp.rot.data(), sp.rot.size() * sizeof(double));
+        cp(r[7] + L.off_occ[p] * sizeof(uint32_t), sp.occ.data(), sp.occ.size() * sizeof(uint32_t));
     };
     const size_t K = pos.size();
     const size_t nth = std::max<size_t>(1, std::min<size_t>(K, std::thread::hardware_concurrency()));
@@ -1224,6 +1169,8 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     }
     CK(ws.pos_elems.ensure(std::max<size_t>(n_elems * sizeof(ElemRec), 16)));
     CK(ws.pos_rot.ensure(std::max<size_t>(n_rot * sizeof(double), 16)));
+    const PosLayout L(pos);
+    CK(ws.pos_occ.ensure(std::max<size_t>(L.b_occ, 16)));
     auto put = [&](DevBuf &dst, size_t off_elems_of_t, const void *src, size_t bytes) -> cudaError_t {
         if (!bytes) return cudaSuccess;
         h2d += bytes;
@@ -1232,11 +1179,10 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     // The positions' tables, staged by stage_positions in page-locked memory laid out as on the
     // device, go over with one copy per array; otherwise each position's arrays are copied from
     // its own vectors.
-    const PosLayout L(pos);
     const bool staged = slot >= 0 && slot <= 1 && ws.pos_host[slot] && ws.pos_staged_k[slot] == K &&
                         ws.pos_staged_bytes[slot] == L.b_all && L.b_all > 0 && L.all_exact == all_exact;
     if (staged) {
-        char *r[7];
+        char *r[8];
         L.regions(static_cast<char *>(ws.pos_host[slot]), r);
         ws.pos_dma_pending[slot] = true;
         CK(put(ws.pos_cells, 0, r[0], L.b_cells));
@@ -1248,6 +1194,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
             CK(put(ws.pos_xc, 0, r[5], L.b_disc));
         }
         CK(put(ws.pos_rot, 0, r[6], L.b_rot));
+        CK(put(ws.pos_occ, 0, r[7], L.b_occ));
     }
     for (size_t p = 0; p < K; ++p) {
         const SunPosition &sp = pos[p];
@@ -1262,6 +1209,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 CK(put(ws.pos_xc, od, sp.cell_xc.data(), nd));
             }
             CK(put(ws.pos_rot, off_rot[p] * sizeof(double), sp.rot.data(), sp.rot.size() * sizeof(double)));
+            CK(put(ws.pos_occ, L.off_occ[p] * sizeof(uint32_t), sp.occ.data(), sp.occ.size() * sizeof(uint32_t)));
         }
         if (!sp.rot.empty()) {
             // the scene's element table (already on the device) copied, then the re-aimed
@@ -1332,6 +1280,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         S.sun.cell_xa = all_exact ? ws.pos_xa.as<float4>() + off_disc[p] : nullptr;
         S.sun.cell_xb = all_exact ? ws.pos_xb.as<float4>() + off_disc[p] : nullptr;
         S.sun.cell_xc = all_exact ? ws.pos_xc.as<float4>() + off_disc[p] : nullptr;
+        S.sun.occ = ws.pos_occ.as<uint32_t>() + L.off_occ[p];
         S.sun.inv_cdf = hs.inv_cdf.empty() ? nullptr : ws.inv_cdf.as<double>();
         if (off_elems[p] != size_t(-1)) S.elems = ws.pos_elems.as<ElemRec>() + off_elems[p];
         S.seed = pos[p].seed;
@@ -1386,9 +1335,6 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         CK(ws.etotal.ensure(8));
         CK(wf_buffers(ws, S0, n, W, Q));
     }
-    Workspace::Tuning &tu = ws.tune[rq.precision ? 1 : 0];
-    if (!tu.done) CK(autotune(ws, Sp[0], rq.precision, rq.max_sun, st, out.gpu_launches));
-    out.probe_variant = tu.probe;
     CK(cudaStreamSynchronize(st));
     out.setup_ms = ms_since(t_setup);
 
@@ -1444,9 +1390,9 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 CK(cudaEventRecord(p0, st));
                 const uint64_t s0 = sun_next[p];
                 if (rq.precision)
-                    out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs + p, tu.probe, st);
+                    out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs + p, st);
                 else
-                    out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs + p, tu.probe, st);
+                    out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs + p, st);
                 launch_scan(po.block_counts, nb, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(),
                             ws.scan_parts.as<uint32_t>(), st);
                 launch_list_sort(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p, n_elem0,

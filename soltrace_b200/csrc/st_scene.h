@@ -23,6 +23,7 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxFluxMaps = 8;
 constexpr int kSunCdfCells = 4096;
 constexpr int kSunInvCells = 8192;
+constexpr int kMaxOccWords = 16384;  // occupancy bitmap of the sun-plane grid: at most 64 KB
 
 // surface model codes after coretrace/input.cpp:288-366 translation
 enum SurfType : int {
@@ -123,21 +124,32 @@ struct SunDev {
     int grid_on, gnx, gny;
     double gx0, gy0, ginv;          // origin and 1/cell size
     const int *cell_start;          // (start, end) per cell: cell c at [2c, 2c+1], read as int2
-    const float4 *cell_disc;        // per cell entry, ascending element order: projected
+    const float4 *cell_disc;        // per cell entry (elements that can accept a hit in the cell),
+                                    // ascending element order: projected
                                     // centre x, y, radius, element index (int bits)
     const float4 *cell_par;         // per cell entry: rows (a, b), (c, d) of the footprint's
                                     // dual basis; (x, y) about the centre is kept when
                                     // |a x + b y| <= 1 and |c x + d y| <= 1 (all zero: disc only)
     double gcell;                   // cell size (1 / ginv)
     // first stages of flat rectangles only (exact_flat), per cell entry: the footprint centre
-    // relative to the cell's lower corner, the padded disc radius squared and the element
-    // (xa); the exact footprint's dual basis rows, unpadded (xb); the depth slopes along the
-    // sun's z and the depth at the centre (xc; z +inf: the element accepts no hit, NaN: no
-    // exact footprint, the float test defers to double)
+    // relative to the cell's lower corner, the depth's margin and the element (xa); the exact
+    // footprint's dual basis rows, unpadded (xb); the depth slopes along the sun's z, the depth at
+    // the centre and the margin of the footprint test (xc; +inf: no exact footprint, always
+    // decided in double)
     int exact_flat;
-    const float4 *cell_xa;          // centre x, y (cell-relative), r^2, element (int bits)
+    float fcell;                    // gcell
+    // sun-plane point in fixed point: with U the top 32 bits of a coordinate's uniform variate,
+    // U * mul = (cells from the lower edge) * 2^(32 + shift)
+    uint32_t fx_mul, fy_mul;
+    int fx_shift, fy_shift;
+    // occupancy bitmap, finer or coarser than the cells by a power of two: bit (ix, iy), ix the
+    // high word of U * mul shifted right by occ_shx, is set where a footprint may lie; rows of
+    // occ_stride words
+    int occ_shx, occ_shy, occ_stride, occ_words;
+    const uint32_t *occ;
+    const float4 *cell_xa;          // centre x, y (cell-relative), depth margin, element (int bits)
     const float4 *cell_xb;          // i00, i01, i10, i11
-    const float4 *cell_xc;          // dz/dx, dz/dy, z at the centre, unused
+    const float4 *cell_xc;          // dz/dx, dz/dy, z at the centre, footprint margin
 };
 
 struct SceneDev {

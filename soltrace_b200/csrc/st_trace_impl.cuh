@@ -676,140 +676,7 @@ __global__ void __launch_bounds__(kResolveBlock, MINB) k_sun_resolve(const __gri
     }
 }
 
-// Mixed-precision probe of sun rays on a first stage of flat rectangles (SunDev::exact_flat)
-// in one kernel.  Each grid entry whose padded disc holds the sun-plane point is tested
-// against the element's exact footprint and plane in float: inside the rectangle when
-// |u|, |v| <= 1 for (u, v) the point in the projected half-axes' basis, at depth
-// z0 + gx qx + gy qy along the sun's z (the nearest accepted element wins, as the path
-// lengths of raytrace.cpp:745 order them).  A point within the float rounding margins of a
-// footprint edge, an entry without an exact footprint, or two accepted elements within
-// rounding of one depth leave the ray undecided: it goes to a list that k_sun_resolve_amb
-// searches in double, so the element found is the FP64 probe's.  Output as k_sun_resolve
-// leaves it: hitting rays listed with their element, one hit-mask bit per ray, hits per
-// kProbeBlock rays.  RPT sun rays per thread at kProbeBlock apart (4, 8 or 16: the autotuner's
-// variants), RPT x kProbeBlock per block.
-template <int MIXED, int RPT>
-__global__ void __launch_bounds__(kProbeBlock, kExactProbeMinBlocks) k_sun_probe_exact(const __grid_constant__ SceneDev S, uint64_t s0,
-                                                                  uint32_t n, ProbeOut o, const RunState *rs) {
-    const uint32_t nb = (n + kProbeBlock - 1) / kProbeBlock;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (rs->reached) {  // the requested hits are numbered: this batch is surplus
-        if (threadIdx.x < RPT && blockIdx.x * RPT + threadIdx.x < nb)
-            o.block_counts[blockIdx.x * RPT + threadIdx.x] = 0;
-        if (o.hit_mask && threadIdx.x < (RPT * kProbeBlock) / 32) o.hit_mask[blockIdx.x * ((RPT * kProbeBlock) / 32) + threadIdx.x] = 0;
-        return;
-    }
-    const SunDev &sun = S.sun;
-    // per ray of the block its result, per warp and ray group the hit ballot
-    constexpr uint32_t kUndecided = 0xffffffffu;
-    __shared__ uint32_t hsh[RPT][kProbeBlock];
-    __shared__ unsigned wb[RPT][kProbeBlock / 32];
-    __shared__ uint32_t wn[kProbeBlock / 32], base;
-    // pass 1, float only: element + 1, 0 for a miss, kUndecided for the double-precision search
-#pragma unroll 1
-    for (int m = 0; m < RPT; ++m) {
-        const uint32_t i = blockIdx.x * (RPT * kProbeBlock) + m * kProbeBlock + threadIdx.x;
-        uint32_t h = 0;
-        if (i < n) {
-            RayRng rng;
-            rng.init(S.seed, s0 + i, 0);
-            const double xs = sun.xmin + (sun.xmax - sun.xmin) * rng.u();
-            const double ys = sun.ymin + (sun.ymax - sun.ymin) * rng.u();
-            int cx = int(floor((xs - sun.gx0) * sun.ginv)), cy = int(floor((ys - sun.gy0) * sun.ginv));
-            cx = min(max(cx, 0), sun.gnx - 1);
-            cy = min(max(cy, 0), sun.gny - 1);
-            const int2 range = reinterpret_cast<const int2 *>(sun.cell_start)[cy * sun.gnx + cx];
-            // the point relative to the cell's lower corner (entries hold their centres so)
-            const float xr = float(xs - (sun.gx0 + cx * sun.gcell)), yr = float(ys - (sun.gy0 + cy * sun.gcell));
-            int best = -1;
-            float bz = INFINITY;
-            for (int k = range.x; k < range.y; ++k) {
-                const float4 a = sun.cell_xa[k];
-                const float qx = xr - a.x, qy = yr - a.y;
-                if (qx * qx + qy * qy > a.z) continue;  // outside the padded disc
-                const float4 c = sun.cell_xc[k];
-                if (isnan(c.z)) {  // no exact footprint
-                    best = -2;
-                    break;
-                }
-                if (c.z == INFINITY) continue;  // an element that accepts no hit
-                const float4 e0 = sun.cell_xb[k];
-                const float u1 = e0.x * qx, u2 = e0.y * qy, v1 = e0.z * qx, v2 = e0.w * qy;
-                const float au = fabsf(u1 + u2), av = fabsf(v1 + v2);
-                const float mu = 2e-6f * (fabsf(u1) + fabsf(u2)) + 1e-6f;
-                const float mv = 2e-6f * (fabsf(v1) + fabsf(v2)) + 1e-6f;
-                if (au > 1.f + mu || av > 1.f + mv) continue;  // surely outside
-                if (au >= 1.f - mu || av >= 1.f - mv) {         // within rounding of an edge
-                    best = -2;
-                    break;
-                }
-                const float g1 = c.x * qx, g2 = c.y * qy;
-                const float z = c.z + g1 + g2;
-                const float tol = 1e-6f * (fabsf(c.z) + fabsf(g1) + fabsf(g2)) + 1e-5f;
-                if (fabsf(z - bz) <= tol) {  // two elements within rounding of one depth
-                    best = -2;
-                    break;
-                }
-                if (z < bz) {
-                    bz = z;
-                    best = __float_as_int(a.w);
-                }
-            }
-            h = best == -2 ? kUndecided : uint32_t(best + 1);
-        }
-        hsh[m][threadIdx.x] = h;
-    }
-    // pass 2: undecided rays (a few per million) to the double-precision list; ballots, mask
-    uint32_t mine = 0;
-#pragma unroll 1
-    for (int m = 0; m < RPT; ++m) {
-        const uint32_t i = blockIdx.x * (RPT * kProbeBlock) + m * kProbeBlock + threadIdx.x;
-        uint32_t h = hsh[m][threadIdx.x];
-        if (h == kUndecided) {
-            o.amb[atomicAdd(o.amb_count, 1u)] = i;
-            h = 0;
-            hsh[m][threadIdx.x] = 0;
-        }
-        if (o.hit_elem && i < n) o.hit_elem[i] = h;
-        const unsigned bal = __ballot_sync(0xffffffffu, h != 0);
-        if (lane == 0) {
-            if (o.hit_mask) o.hit_mask[(blockIdx.x * (RPT * kProbeBlock) + m * kProbeBlock) / 32 + w] = bal;
-            wb[m][w] = bal;
-        }
-        mine += __popc(bal);
-    }
-    // one reservation in the list per block: warp counts, their prefix, one atomic
-    if (lane == 0) wn[w] = mine;
-    __syncthreads();
-    if (threadIdx.x < RPT && blockIdx.x * RPT + threadIdx.x < nb) {
-        uint32_t c = 0;
-        for (int k = 0; k < kProbeBlock / 32; ++k) c += __popc(wb[threadIdx.x][k]);
-        o.block_counts[blockIdx.x * RPT + threadIdx.x] = c;
-    }
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int k = 0; k < kProbeBlock / 32; ++k) {
-            const uint32_t x = wn[k];
-            wn[k] = t;
-            t += x;
-        }
-        base = t ? atomicAdd(o.cand_count, t) : 0u;
-    }
-    __syncthreads();
-    uint32_t at = base + wn[w];
-    const unsigned lt = (1u << lane) - 1u;
-    for (int m = 0; m < RPT; ++m) {
-        const unsigned bal = wb[m][w];
-        if ((bal >> lane) & 1u) {
-            const uint32_t pos = at + __popc(bal & lt);
-            o.cand[pos] = blockIdx.x * (RPT * kProbeBlock) + m * kProbeBlock + threadIdx.x;
-            if (o.cand_el) o.cand_el[pos] = hsh[m][threadIdx.x];
-        }
-        at += __popc(bal);
-    }
-}
-
-// The rays k_sun_probe_exact left undecided, searched in double (the FP64 probe's arithmetic):
+// The rays k_sun_probe_flat left undecided, searched in double (the FP64 probe's arithmetic):
 // a hit is appended to the probe's list and counted in its block count and hit mask.
 template <int MIXED>
 __global__ void __launch_bounds__(kResolveBlock) k_sun_resolve_amb(const __grid_constant__ SceneDev S, uint64_t s0,
@@ -835,6 +702,253 @@ __global__ void __launch_bounds__(kResolveBlock) k_sun_resolve_amb(const __grid_
 }
 
 #ifdef ST_COMMON_KERNELS
+// Probe of sun rays on a first stage of flat rectangles (SunDev::exact_flat), for both
+// precisions: the float test decides a ray only outside its own rounding margins, and
+// k_sun_resolve_amb searches the rest (a few per million) in the run's double arithmetic, so the
+// element found is the double search's.
+//
+// Every warp takes a contiguous share of the sun rays, in segments of up to kFlatSeg, and runs
+// two steps on its own (blocks only share the bitmap's copy in shared memory):
+//   1. 32 rays: one Philox block each, the sun-plane point in fixed point (SunDev::fx_mul; no
+//      conversions and no double arithmetic) and one bit of the occupancy bitmap.  On a heliostat
+//      field four rays in five end here without a load; the others are queued;
+//   2. once 32 rays are queued (or the segment ends): the entries of each point's grid cell.
+//      Inside an element's rectangle when |u|, |v| <= 1 for (u, v) the point in the projected
+//      half-axes' basis, at depth z0 + gx qx + gy qy along the sun's z; the nearest accepted
+//      element wins, as the path lengths of raytrace.cpp:745 order them.  A point within the
+//      margins of a footprint edge, an entry without an exact footprint, or two accepted
+//      elements within rounding of one depth leave the ray undecided.
+// Output as k_sun_resolve leaves it: hitting rays listed with their element (a reservation per
+// 64 hits or more), one hit-mask bit per ray, hits per kProbeBlock rays.
+//
+// Bound by the issue of integer instructions in step 1 (about 120 a ray, most of them Philox's
+// products and XORs).  A batch of 2^26 sun rays of the 2,000-heliostat field takes 437 us; one
+// thread per ray with the variates converted to double and every ray reading its cell took 620,
+// the double-precision pair k_sun_candidates + k_sun_resolve about 990.  Measured and left: 32
+// warps an SM more (1024-thread blocks at 32 registers) gave the same time.
+//
+// Philox's first three rounds see a counter whose first word is 0 and whose third and fourth
+// are the same for every ray of a segment, so three of their six products are made once a
+// segment (FlatRounds).
+struct FlatRounds {
+    uint32_t a0, b0, c0, d0, e0;  // uniform words of the first rounds
+    uint32_t k0;                  // first key of round 3 (counted from 1)
+};
+__device__ __forceinline__ FlatRounds flat_rounds(uint32_t seed, uint32_t hi) {
+    constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
+    FlatRounds f;
+    uint32_t k0 = seed, k1 = 0x50C7A5E1u;
+    // round 1 of {0, lo, hi, 0x5B200}: words {a0 ^ lo, b, c, 0}
+    f.a0 = __umulhi(M1, hi) ^ k0;
+    const uint32_t b = M1 * hi, c = 0x0005B200u ^ k1;
+    k0 += W0;
+    k1 += W1;
+    // round 2: p = M0 (a0 ^ lo): words {b0, c0, hi(p) ^ d0, lo(p)}
+    f.b0 = __umulhi(M1, c) ^ b ^ k0;
+    f.c0 = M1 * c;
+    f.d0 = k1;
+    k0 += W0;
+    k1 += W1;
+    // round 3: word 2 is hi(M0 b0) ^ lo(p) ^ k1, word 3 lo(M0 b0)
+    f.e0 = __umulhi(M0, f.b0) ^ k1;
+    f.b0 = M0 * f.b0;
+    f.k0 = k0;
+    return f;
+}
+// 32 x 32 -> 64-bit product in one instruction (__umulhi and the low product take two)
+__device__ __forceinline__ void mul_wide(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo) {
+    const uint64_t p = uint64_t(a) * b;
+    hi = uint32_t(p >> 32);
+    lo = uint32_t(p);
+}
+// the top 32 bits of the first two variates (words_to_unit) of the rays whose stream indices have
+// low words lo and lo + 32 (and the segment's high word): two independent chains in flight
+__device__ __forceinline__ void flat_variates(const FlatRounds &f, const FlatKeys &key, uint32_t lo, uint32_t ux[2],
+                                              uint32_t uy[2]) {
+    constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u;
+    uint32_t c0[2], c1[2], c2[2], c3[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        uint32_t h, l, y;
+        mul_wide(M0, f.a0 ^ (lo + 32u * r), h, l);
+        y = h ^ f.d0;
+        mul_wide(M1, y, h, c1[r]);
+        c0[r] = h ^ f.c0 ^ f.k0;
+        c2[r] = f.e0 ^ l;
+        c3[r] = f.b0;
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            uint32_t h0, l0, h1, l1;
+            mul_wide(M0, c0[r], h0, l0);
+            mul_wide(M1, c2[r], h1, l1);
+            c0[r] = h1 ^ c1[r] ^ key.k0[q];
+            c1[r] = l1;
+            c2[r] = h0 ^ c3[r] ^ key.k1[q];
+            c3[r] = l0;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        ux[r] = (c0[r] & ~31u) | (c1[r] >> 27);
+        uy[r] = (c2[r] & ~31u) | (c3[r] >> 27);
+    }
+}
+// the same for two rays of any stream indices (a segment that crosses a 2^32 boundary)
+__device__ __noinline__ uint4 flat_variates_any(uint32_t seed, uint64_t sid) {
+    uint32_t v[4];
+    for (int r = 0; r < 2; ++r, sid += 32) {
+        uint32_t w0 = 0, w1 = uint32_t(sid), w2 = uint32_t(sid >> 32), w3 = 0x0005B200u;
+        philox10(w0, w1, w2, w3, seed, 0x50C7A5E1u);
+        v[2 * r] = (w0 & ~31u) | (w1 >> 27);
+        v[2 * r + 1] = (w2 & ~31u) | (w3 >> 27);
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+struct FlatWarp {                  // a warp's shared memory
+    uint2 q[kFlatQueue];           // queued rays: 32-bit variates; the last slot takes the others' stores
+    uint2 hits[kFlatHits];         // hits to list: ray of the batch, element + 1
+    uint32_t mask[kFlatSeg / 32];  // the segment's hit bits
+    uint16_t qi[kFlatQueue];       // queued rays: place in the segment
+};
+static_assert(sizeof(FlatWarp) == kFlatWarpBytes, "sized by the launcher");
+__global__ void __launch_bounds__(kFlatBlock, 2) k_sun_probe_flat(const __grid_constant__ SceneDev S,
+                                                                  const __grid_constant__ FlatKeys keys, uint64_t s0,
+                                                                  uint32_t n, ProbeOut o, const RunState *rs) {
+    const SunDev &sun = S.sun;
+    extern __shared__ __align__(16) unsigned char flat_sh[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    constexpr int kWarps = kFlatBlock / 32, kUnit = kProbeBlock, kSegUnits = kFlatSeg / kUnit;
+    FlatWarp &sh = reinterpret_cast<FlatWarp *>(flat_sh)[warp];
+    uint32_t *occ = reinterpret_cast<uint32_t *>(flat_sh + kWarps * sizeof(FlatWarp));
+    // this warp's units of kProbeBlock rays
+    const uint32_t nb = (n + kUnit - 1) / kUnit;
+    const uint64_t w = uint64_t(blockIdx.x) * kWarps + warp, W = uint64_t(gridDim.x) * kWarps;
+    const uint32_t u0 = uint32_t(nb * w / W), u1 = uint32_t(nb * (w + 1) / W);
+    if (rs->reached) {  // the requested hits are numbered: this batch is surplus
+        for (uint32_t u = u0; u < u1; ++u) {
+            if (lane == 0) o.block_counts[u] = 0;
+            if (lane < kUnit / 32) o.hit_mask[u * (kUnit / 32) + lane] = 0;
+        }
+        return;
+    }
+    for (int k = threadIdx.x; k < sun.occ_words; k += kFlatBlock) occ[k] = sun.occ[k];
+    __syncthreads();
+    uint32_t nh = 0;
+    auto list_hits = [&]() {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(o.cand_count, nh);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (uint32_t k = lane; k < nh; k += 32) {
+            const uint2 h = sh.hits[k];
+            o.cand[base + k] = h.x;
+            o.cand_el[base + k] = h.y;
+        }
+        nh = 0;
+        __syncwarp();
+    };
+    for (uint32_t u = u0; u < u1; u += kSegUnits) {
+        const int units = min(uint32_t(kSegUnits), u1 - u);
+        const uint32_t t0 = u * kUnit;
+        const int last = units * kUnit;
+        const uint64_t sid0 = s0 + t0;
+        const FlatRounds fr = flat_rounds(S.seed, uint32_t(sid0 >> 32));
+        const bool crosses = uint32_t(sid0) > 0xffffffffu - uint32_t(kFlatSeg - 1);  // a segment over a 2^32 boundary
+        for (int k = lane; k < kFlatSeg / 32; k += 32) sh.mask[k] = 0;
+        int nq = 0;
+        __syncwarp();
+        const uint32_t lim = n - t0;
+#pragma unroll 1
+        for (int m = 0; m < last; m += 64) {
+            // ---- step 1: 64 rays ----
+            uint32_t ux[2], uy[2];
+            if (!crosses) {
+                flat_variates(fr, keys, uint32_t(sid0) + m + lane, ux, uy);
+            } else {
+                const uint4 v = flat_variates_any(S.seed, sid0 + m + lane);
+                ux[0] = v.x;
+                uy[0] = v.y;
+                ux[1] = v.z;
+                uy[1] = v.w;
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint32_t j = m + lane + 32 * r;
+                const uint32_t ix = __umulhi(ux[r], sun.fx_mul) >> sun.occ_shx,
+                               iy = __umulhi(uy[r], sun.fy_mul) >> sun.occ_shy;
+                const uint32_t bit = (occ[iy * sun.occ_stride + (ix >> 5)] >> (ix & 31)) & uint32_t(j < lim);
+                const unsigned bal = __ballot_sync(0xffffffffu, bit & 1u);
+                // every lane stores (no branch): the lanes without a queued ray into the spare slot
+                const int at = (bit & 1u) ? nq + __popc(bal & lt) : kFlatQueue - 1;
+                sh.q[at] = make_uint2(ux[r], uy[r]);
+                sh.qi[at] = uint16_t(j);
+                nq += __popc(bal);
+            }
+            __syncwarp();
+#pragma unroll 1
+            while (nq >= 32 || (nq > 0 && m + 64 >= last)) {
+                // ---- step 2: the last 32 queued rays ----
+                const int first = max(nq - 32, 0), c = first + lane;
+                int best = -1;  // element, -1 a miss
+                bool undecided = false;
+                uint32_t j = 0;
+                if (c < nq) {
+                    const uint2 v = sh.q[c];
+                    j = sh.qi[c];
+                    uint32_t hx, hy, bx, by;
+                    mul_wide(v.x, sun.fx_mul, hx, bx);
+                    mul_wide(v.y, sun.fy_mul, hy, by);
+                    const int2 range = reinterpret_cast<const int2 *>(
+                        sun.cell_start)[(hy >> sun.fy_shift) * sun.gnx + (hx >> sun.fx_shift)];
+                    bx = __funnelshift_r(bx, hx, sun.fx_shift + 9);
+                    by = __funnelshift_r(by, hy, sun.fy_shift + 9);
+                    // the point relative to the cell's lower corner (entries hold their centres so)
+                    const float xr = (__uint_as_float(0x3f800000u | (bx & 0x7fffffu)) - 1.0f) * sun.fcell;
+                    const float yr = (__uint_as_float(0x3f800000u | (by & 0x7fffffu)) - 1.0f) * sun.fcell;
+                    float bz = INFINITY, bt = 0.f;
+#pragma unroll 1
+                    for (int k = range.x; k < range.y; ++k) {
+                        const float4 a = sun.cell_xa[k], e = sun.cell_xb[k], g = sun.cell_xc[k];
+                        const float qx = xr - a.x, qy = yr - a.y;
+                        const float t = fmaxf(fabsf(e.x * qx + e.y * qy), fabsf(e.z * qx + e.w * qy));
+                        const float z = g.z + g.x * qx + g.y * qy;
+                        const bool in = t < 1.f - g.w;  // surely inside; else undecided unless surely outside
+                        undecided = undecided || !(in || t > 1.f + g.w) || (in && fabsf(z - bz) <= a.z + bt);
+                        if (in && z < bz) {
+                            bz = z;
+                            bt = a.z;
+                            best = __float_as_int(a.w);
+                        }
+                    }
+                    if (undecided) {
+                        best = -1;
+                        o.amb[atomicAdd(o.amb_count, 1u)] = t0 + j;
+                    }
+                    if (best >= 0) atomicOr(&sh.mask[j >> 5], 1u << (j & 31));
+                }
+                nq = first;
+                const unsigned bal = __ballot_sync(0xffffffffu, best >= 0);
+                if (best >= 0) sh.hits[nh + __popc(bal & lt)] = make_uint2(t0 + j, uint32_t(best + 1));
+                nh += __popc(bal);
+                __syncwarp();
+                if (nh > kFlatHits - 32) list_hits();
+            }
+        }
+        if (lane < units * (kUnit / 32)) o.hit_mask[u * (kUnit / 32) + lane] = sh.mask[lane];
+        if (lane < units) {
+            uint32_t c = 0;
+            for (int k = 0; k < kUnit / 32; ++k) c += __popc(sh.mask[lane * (kUnit / 32) + k]);
+            o.block_counts[u + lane] = c;
+        }
+        __syncwarp();
+    }
+    if (nh) list_hits();
+}
+
 // first kernel of the grid probe (above): candidates listed, hit-mask words cleared
 __global__ void __launch_bounds__(kProbeBlock) k_sun_candidates(const __grid_constant__ SceneDev S, uint64_t s0,
                                                                 uint32_t n, ProbeOut o, const RunState *rs) {
