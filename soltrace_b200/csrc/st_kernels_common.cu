@@ -38,11 +38,16 @@ bool launch_sun_probe_flat(const SceneDev &S, uint64_t s0, uint32_t n, const Pro
 void launch_offsets(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, cudaStream_t st) {
     k_offsets<<<1, 1024, 0, st>>>(counts, nb, offsets, total);
 }
-void launch_scan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, uint32_t *parts,
-                 cudaStream_t st) {
+int launch_scan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, uint32_t *parts,
+                cudaStream_t st) {
+    if (nb <= kScanOneBlock) {
+        k_offsets<<<1, 1024, 0, st>>>(counts, nb, offsets, total);
+        return 1;
+    }
     const uint32_t chunks = std::max(1u, (nb + kScanChunk - 1) / kScanChunk);
     k_scan_parts<<<chunks, kScanBlock, 0, st>>>(counts, nb, parts);
     k_scan_chunks<<<chunks, kScanBlock, 0, st>>>(counts, nb, parts, offsets, total);
+    return 2;
 }
 // chunk scans from the scanned chunk sums (k_scan_chunks with the sum of the chunks before
 // each read instead of added up)
@@ -165,6 +170,11 @@ void launch_compact(uint64_t s0, uint32_t n, const uint32_t *hit_elem, const uin
 void launch_advance(const uint32_t *total, const uint64_t *hit_sid, uint64_t s0, uint32_t n, RunState *rs,
                     cudaStream_t st) {
     k_advance<<<1, 1, 0, st>>>(total, hit_sid, s0, n, rs);
+}
+void launch_list_rank(uint64_t s0, const ProbeOut &o, const uint32_t *offsets, const uint32_t *total, RunState *rs,
+                      HitRec *hits, uint32_t max_n, cudaStream_t st) {
+    const uint32_t blocks = std::max(1u, std::min<uint32_t>((max_n + 255) / 256, 148u * 8u));
+    k_list_rank<<<blocks, 256, 0, st>>>(s0, o, offsets, total, rs, hits);
 }
 void launch_list_sort(uint64_t s0, const ProbeOut &o, const uint32_t *offsets, const uint32_t *total, RunState *rs,
                       uint32_t n_elem0, uint32_t *elem_count, uint32_t *elem_cursor, uint32_t *scratch_total,

@@ -99,7 +99,7 @@ struct WfQueues {
     uint32_t *shade;
     uint32_t *counts;                     // (rounds + 1) * (n_queues + 1) entries
     uint32_t cap;
-    int rounds;
+    int rounds;                           // 0: the finishing kernel takes the rays from the first kernel
     int n_queues;
     int queue_kind[kMaxStages];           // search kind of queue k
     unsigned char stage_queue[kMaxStages];  // search queue of the rays of stage s
@@ -190,14 +190,28 @@ int launch_trace_mixed(bool records, const SceneDev &S, const HitRec *hits, cons
 void launch_list_sort(uint64_t s0, const ProbeOut &o, const uint32_t *offsets, const uint32_t *total, RunState *rs,
                       uint32_t n_elem0, uint32_t *elem_count, uint32_t *elem_cursor, uint32_t *scratch_total,
                       HitRec *hits, uint32_t max_n, cudaStream_t st);
+// The batch's hits as launch_list_sort leaves them, in sun-ray order instead: one kernel for
+// batches whose numbered rays fit the GPU at once (small_batch)
+void launch_list_rank(uint64_t s0, const ProbeOut &o, const uint32_t *offsets, const uint32_t *total, RunState *rs,
+                      HitRec *hits, uint32_t max_n, cudaStream_t st);
+// A batch that numbers at most kSmallRays rays is traced by the first and the finishing kernel
+// alone (no rounds): every ray has a thread of its own from start to end, and what the rounds'
+// full warps save is less than their launches cost.  The line lies below the 75,776 threads the
+// finishing kernel keeps resident: device time of a run in us, rounds and sort against this path:
+// dish 163 to 82 at 1,000 hits and 195 to 94 at 65,536, trough 323 to 180, 2,000-heliostat field
+// 215 to 139, beam-down tower 330 to 201; at 130,000 hits the trough would go from 383 to 569
+// (a thread's second ray waits for the longest first one of its warp).
+constexpr uint64_t kSmallRays = 65536;
 // finite-element interpolation failures flagged by the kernels since the last call
 unsigned take_fe_failures_fp64();
 unsigned take_fe_failures_mixed();
 void launch_offsets(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, cudaStream_t st);
-// the same exclusive scan over the whole grid (two kernels); `parts` holds scan_parts(nb)
-// chunk sums
-void launch_scan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, uint32_t *parts,
-                 cudaStream_t st);
+// the same exclusive scan over the whole grid (two kernels; one block scans up to kScanOneBlock
+// counts in the time of one of them); `parts` holds scan_parts(nb) chunk sums.  Returns the
+// number of kernels launched.
+int launch_scan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *total, uint32_t *parts,
+                cudaStream_t st);
+constexpr uint32_t kScanOneBlock = 8192;
 constexpr int kScanChunk = 2048, kScanBlock = 256;
 constexpr size_t scan_parts(uint32_t nb) { return (size_t(nb) + kScanChunk - 1) / kScanChunk + 1; }
 // the same scan for arrays of any length (up to 2^31 entries): chunk sums, their scan, and

@@ -696,6 +696,9 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 return false;
             }
             uint64_t queued = 0;
+            // the rays still to be numbered when the group was planned bound those of each of its batches
+            const uint64_t batch_most =
+                explicit_mode ? want : rq.n_hits - std::min<uint64_t>(rq.n_hits, multi ? global_done : rs.hits_done);
             while (queued < want) {
                 // this batch's global sun-ray range [sun_next, sun_next + n_all) and, over several
                 // ranks, this rank's contiguous slice [s0, s0 + n) of it
@@ -730,9 +733,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                         out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs, st);
                     else
                         out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs, st);
-                    launch_scan(po.block_counts, nb, d_offsets.as<uint32_t>(), d_total.as<uint32_t>(),
-                                ws.scan_parts.as<uint32_t>(), st);
-                    out.gpu_launches += 2;
+                    out.gpu_launches += launch_scan(po.block_counts, nb, d_offsets.as<uint32_t>(), d_total.as<uint32_t>(),
+                                                    ws.scan_parts.as<uint32_t>(), st);
                 } else {
                     CK(cudaMemsetAsync(d_total.p, 0, 8, st));
                 }
@@ -764,7 +766,13 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                     out.h2d_bytes += sizeof rs;
                     global_done += std::min<uint64_t>(all, rq.n_hits - global_done);
                 }
-                if (n > 0) {
+                // rays this batch can number: what the small-batch rule goes by
+                const bool small = std::min<uint64_t>(n, batch_most) <= kSmallRays;
+                if (n > 0 && small) {
+                    launch_list_rank(s0, po, d_offsets.as<uint32_t>(), d_total.as<uint32_t>(), drs, d_s_hits.as<HitRec>(),
+                                     uint32_t(n), st);
+                    out.gpu_launches += 1;
+                } else if (n > 0) {
                     launch_list_sort(s0, po, d_offsets.as<uint32_t>(), d_total.as<uint32_t>(), drs, n_elem0,
                                      d_ecount.as<uint32_t>(), d_ecursor.as<uint32_t>(), d_etotal.as<uint32_t>(),
                                      d_s_hits.as<HitRec>(),
@@ -776,6 +784,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 WfState W;
                 WfQueues Q;
                 CK(wf_buffers(ws, S, n, W, Q));
+                if (small) Q.rounds = 0;
                 CK(save_setup(n));
                 CK(cudaEventRecord(p1, st));
                 if (n > 0) {
@@ -1393,12 +1402,20 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                     out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs + p, st);
                 else
                     out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs + p, st);
-                launch_scan(po.block_counts, nb, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(),
-                            ws.scan_parts.as<uint32_t>(), st);
-                launch_list_sort(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p, n_elem0,
-                                 ws.ecount.as<uint32_t>(), ws.ecursor.as<uint32_t>(), ws.etotal.as<uint32_t>(),
-                                 ws.s_hits.as<HitRec>(),
-                                 uint32_t(n), st);
+                out.gpu_launches += launch_scan(po.block_counts, nb, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(),
+                                                ws.scan_parts.as<uint32_t>(), st);
+                if (std::min<uint64_t>(n, need) <= kSmallRays) {
+                    launch_list_rank(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p,
+                                     ws.s_hits.as<HitRec>(), uint32_t(n), st);
+                    out.gpu_launches += 1;
+                    Q.rounds = 0;
+                } else {
+                    launch_list_sort(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p, n_elem0,
+                                     ws.ecount.as<uint32_t>(), ws.ecursor.as<uint32_t>(), ws.etotal.as<uint32_t>(),
+                                     ws.s_hits.as<HitRec>(),
+                                     uint32_t(n), st);
+                    out.gpu_launches += 3;
+                }
                 CK(cudaEventRecord(p1, st));
                 if (rq.precision)
                     out.gpu_launches += launch_trace_mixed(false, S, ws.s_hits.as<HitRec>(), ws.total.as<uint32_t>(), drs + p,
@@ -1409,7 +1426,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 CK(cudaEventRecord(p2, st));
                 launch_advance(ws.total.as<uint32_t>(), nullptr, s0, uint32_t(n), drs + p, st);
                 CK(cudaGetLastError());
-                out.gpu_launches += 6;  // scan (two kernels), sort (three), advance
+                out.gpu_launches += 1;
                 probe_ev.push_back({p0, p1});
                 trace_ev.push_back({p1, p2});
                 queued += n;

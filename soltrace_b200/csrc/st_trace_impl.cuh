@@ -1285,6 +1285,19 @@ __global__ void __launch_bounds__(kSortBlock) k_list_scatter_sh(uint64_t s0, Pro
     }
 }
 
+// A small batch's hits in sun-ray order, unsorted: each goes to the place of its rank.
+__global__ void __launch_bounds__(256) k_list_rank(uint64_t s0, ProbeOut o, const uint32_t *offsets,
+                                                   const uint32_t *total, RunState *rs, HitRec *hits) {
+    const uint32_t n = *o.cand_count;
+    const uint32_t take = batch_take(rs, total);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const uint32_t h = o.cand_el[i];
+        if (!h) continue;
+        const uint32_t ray = o.cand[i], rank = rank_of(rank_load(offsets, o.hit_mask, ray), ray);
+        list_put(s0, ray, h - 1, rank, rank, take, rs, hits);
+    }
+}
+
 // single thread: apply the cut-off at the requested hit count and advance the run state
 __global__ void k_advance(const uint32_t *total, const uint64_t *hit_sid, uint64_t s0, uint32_t n, RunState *rs) {
     rs->cursor = 0;  // the next batch's trace work queue starts empty
@@ -1835,23 +1848,26 @@ __global__ void __launch_bounds__(kTraceBlock, CLOSED ? (MIXED ? kWfClosedShadeM
     wf_ctr_flush(c, S, O);
 }
 
-// Finishing kernel: every ray still queued (the search queues of round `rounds`) runs to
-// its end, one step after the other.
-template <int MIXED, int RECORDS>
+// Finishing kernel: every ray still queued (round `rounds`'s queues) runs to its end, one step
+// after the other.  CLOSED: every stage has closed-form surfaces only.
+template <int MIXED, int RECORDS, int CLOSED>
 __global__ void __launch_bounds__(kTraceBlock, kWfShadeMinBlocks) k_wf_finish(const __grid_constant__ SceneDev S, TraceOut O,
                                                                               WfState W, const __grid_constant__ WfQueues Q) {
     __shared__ WfBlockCtr c;
     wf_ctr_init(c);
     const int nq = Q.n_queues, R = Q.rounds;
     const uint32_t *cnt = Q.counts + R * (nq + 1);
-    for (int k = 0; k < nq; ++k) {
+    // the search queues, then the shade queue (rays the first kernel searched itself, when no
+    // round was launched)
+    for (int k = 0; k <= nq; ++k) {
         const uint32_t n = cnt[k];
-        const uint32_t *q_in = Q.search[R & 1] + size_t(k) * Q.cap;
+        const uint32_t *q_in = k < nq ? Q.search[R & 1] + size_t(k) * Q.cap : Q.shade;
         for (uint32_t q = blockIdx.x * kTraceBlock + threadIdx.x; q < n; q += gridDim.x * kTraceBlock) {
             WfRay r = wf_load(W, q_in[q]);
             int status = (r.next_j >= 0) ? int(kWfShade) : int(kWfSearch);
             while (status != kWfDone)
-                status = (status == kWfShade) ? wf_shade<MIXED, RECORDS>(S, O, c, r) : wf_search<MIXED, RECORDS>(S, O, c, r);
+                status = (status == kWfShade) ? wf_shade<MIXED, RECORDS, 0, CLOSED>(S, O, c, r)
+                                              : wf_search<MIXED, RECORDS, CLOSED ? kSearchClosed : 0>(S, O, c, r);
         }
     }
     wf_ctr_flush(c, S, O);
@@ -1875,14 +1891,15 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
                      const uint32_t *total, const RunState *rs, const TraceOut &O, const WfState &W,
                      const WfQueues &Q, const ReplayIn *replay, cudaStream_t st) {
     // persistent grids: every block the kernels can keep resident on every SM
-    static int per_sm[6] = {0, 0, 0, 0, 0, 0};
+    static int per_sm[7] = {0, 0, 0, 0, 0, 0, 0};
     if (per_sm[0] == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_wf_first<MIXED, RECORDS, 0>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[4], k_wf_first<MIXED, RECORDS, 1>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[5], k_wf_first<MIXED, RECORDS, 2>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_wf_shade<MIXED, RECORDS, 0>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[3], k_wf_shade<MIXED, RECORDS, 1>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_wf_finish<MIXED, RECORDS>, kTraceBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_wf_finish<MIXED, RECORDS, 0>, kTraceBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[6], k_wf_finish<MIXED, RECORDS, 1>, kTraceBlock, 0);
         for (int &x : per_sm) x = x > 0 ? x : 1;
     }
     int dev = 0, sms = 148;
@@ -1922,7 +1939,10 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
             k_wf_shade<MIXED, RECORDS, 0><<<sms * per_sm[1], kTraceBlock, 0, st>>>(S, O, W, Q, r);
         ++launches;
     }
-    k_wf_finish<MIXED, RECORDS><<<sms * per_sm[2], kTraceBlock, 0, st>>>(S, O, W, Q);
+    if (all_closed)
+        k_wf_finish<MIXED, RECORDS, 1><<<sms * per_sm[6], kTraceBlock, 0, st>>>(S, O, W, Q);
+    else
+        k_wf_finish<MIXED, RECORDS, 0><<<sms * per_sm[2], kTraceBlock, 0, st>>>(S, O, W, Q);
     return launches;
 }
 
