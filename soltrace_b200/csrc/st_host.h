@@ -32,6 +32,8 @@ struct HostScene {
     std::vector<uint32_t> occ;  // occupancy bitmap of the exact flat footprints (SunDev)
     std::vector<double> inv_cdf;  // table-sunshape inverse CDF (kSunInvCells + 1 entries)
     SceneDev dev;  // stages, sun scalars and flags; device pointers are filled by gpu_run
+    uint64_t version = 0;  // another number for every flattened scene of the process, 0: none given
+    bool has_fe = false;   // an element has a finite-element surface (its queries can fail)
 };
 
 struct FluxMapReq {
@@ -47,7 +49,8 @@ struct RunRequest {
     int precision = 0;
     bool records = true;
     int device = 0;
-    std::vector<double> ex_pos, ex_cos;  // explicit rays (global frame)
+    uint64_t n_explicit = 0;             // explicit rays (global frame), held by the caller
+    const double *ex_pos = nullptr, *ex_cos = nullptr;
     std::vector<FluxMapReq> flux;
     int (*callback)(unsigned long, unsigned long, unsigned long, unsigned long, unsigned long, void *) = nullptr;
     void *cbdata = nullptr;

@@ -109,8 +109,27 @@ struct Workspace {
     DevBuf pos_cells, pos_disc, pos_par, pos_xa, pos_xb, pos_xc, pos_occ, pos_elems, pos_rot, pos_rs, pos_ctr, pos_acc;
     DevBuf cell_xa, cell_xb, cell_xc, occ;  // exact flat footprints of the sun-plane grid
     std::vector<cudaEvent_t> events;
+    // the scene whose tables the buffers above hold (HostScene::version), 0 for none: a run on
+    // the same scene copies nothing of it again
+    uint64_t scene_version = 0;
+    // page-locked landing place of what the host reads back per batch, so that one wait covers all
+    struct Mail {
+        RunState rs;
+        RunCounters ctr;
+        unsigned long long nrec, stage_records[kMaxStages];
+        unsigned int bad;
+    } *mail = nullptr;
+    unsigned long long *acc_host = nullptr;  // the same for accumulators of up to kAccHost values
+    static constexpr size_t kAccHost = 1u << 16;
+    cudaError_t mailbox() {
+        cudaError_t e = mail ? cudaSuccess : cudaMallocHost(&mail, sizeof(Mail));
+        if (e == cudaSuccess && !acc_host) e = cudaMallocHost(&acc_host, kAccHost * sizeof(unsigned long long));
+        return e;
+    }
     ~Workspace() {
         if (device >= 0) cudaSetDevice(device);
+        if (mail) cudaFreeHost(mail);
+        if (acc_host) cudaFreeHost(acc_host);
         for (int k = 0; k < 2; ++k)
             if (pos_host[k]) cudaFreeHost(pos_host[k]);
         if (rec_host) {
@@ -270,10 +289,10 @@ static std::string order_records(Workspace &ws, const RecordDev *recs, unsigned 
     cudaMemsetAsync(o.stage_count, 0, kMaxStages * 8, st);
     cudaMemsetAsync(o.bad, 0, 8, st);
     if (nrec) launch_rec_count(o, st);
-    unsigned long long cnt[kMaxStages] = {0};
-    unsigned int bad = 0;
-    cudaMemcpyAsync(cnt, o.stage_count, kMaxStages * 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&bad, o.bad, 4, cudaMemcpyDeviceToHost, st);
+    const unsigned long long *cnt = ws.mail->stage_records;
+    const unsigned int &bad = ws.mail->bad;
+    cudaMemcpyAsync(ws.mail->stage_records, o.stage_count, kMaxStages * 8, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&ws.mail->bad, o.bad, 4, cudaMemcpyDeviceToHost, st);
     // the key slots: exclusive scan of the counts, in place (runs while the host plans the merge)
     launch_scan_large(o.key, uint32_t(nkeys), o.key, ws.rec_bad.as<uint32_t>() + 1, ws.rec_parts.as<uint32_t>(),
                       ws.rec_parts2.as<uint32_t>(), st);
@@ -344,7 +363,7 @@ static std::string order_records(Workspace &ws, const RecordDev *recs, unsigned 
     }
     if (col_bytes && (e = cudaMemcpyAsync(ws.rec_host, ws.rec_cols.p, col_bytes, cudaMemcpyDeviceToHost, st)))
         return std::string("CUDA error: ") + cudaGetErrorString(e);
-    cudaMemcpyAsync(&bad, o.bad, 4, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&ws.mail->bad, o.bad, 4, cudaMemcpyDeviceToHost, st);
     if ((e = cudaStreamSynchronize(st))) return std::string("CUDA error: ") + cudaGetErrorString(e);
     if (bad) return "the records could not be put in order";
     d2h += col_bytes + 8 * kMaxStages + 8;
@@ -394,29 +413,41 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     DevBuf &d_elems = ws.elems, &d_optics = ws.optics, &d_surf = ws.surf, &d_tables = ws.tables, &d_bvh = ws.bvh,
            &d_bvh_items = ws.bvh_items, &d_cell_start = ws.cell_start, &d_cell_disc = ws.cell_disc,
            &d_inv_cdf = ws.inv_cdf, &d_expos = ws.expos, &d_excos = ws.excos;
-    CK(upload(d_elems, hs.elems, st, out.h2d_bytes));
-    CK(upload(ws.elem_sphere, hs.elem_sphere, st, out.h2d_bytes));
-    CK(upload(ws.stage_cells, hs.stage_cells, st, out.h2d_bytes));
-    CK(upload(ws.grid_sphere, hs.grid_sphere, st, out.h2d_bytes));
-    CK(upload(ws.grid_elem, hs.grid_elem, st, out.h2d_bytes));
-    CK(upload(ws.beam_axis, hs.beam_axis, st, out.h2d_bytes));
-    CK(upload(ws.beam_range, hs.beam_range, st, out.h2d_bytes));
-    CK(upload(ws.beam_elem, hs.beam_elem, st, out.h2d_bytes));
-    CK(upload(d_optics, hs.optics, st, out.h2d_bytes));
-    CK(upload(d_surf, hs.surf_data, st, out.h2d_bytes));
-    CK(upload(d_tables, hs.tables, st, out.h2d_bytes));
-    CK(upload(d_bvh, hs.bvh, st, out.h2d_bytes));
-    CK(upload(d_bvh_items, hs.bvh_items, st, out.h2d_bytes));
-    CK(upload(d_cell_start, hs.cell_start, st, out.h2d_bytes));
-    CK(upload(d_cell_disc, hs.cell_disc, st, out.h2d_bytes));
-    CK(upload(ws.cell_par, hs.cell_par, st, out.h2d_bytes));
-    CK(upload(ws.cell_xa, hs.cell_xa, st, out.h2d_bytes));
-    CK(upload(ws.cell_xb, hs.cell_xb, st, out.h2d_bytes));
-    CK(upload(ws.cell_xc, hs.cell_xc, st, out.h2d_bytes));
-    CK(upload(ws.occ, hs.occ, st, out.h2d_bytes));
-    CK(upload(d_inv_cdf, hs.inv_cdf, st, out.h2d_bytes));
-    CK(upload(d_expos, rq.ex_pos, st, out.h2d_bytes));
-    CK(upload(d_excos, rq.ex_cos, st, out.h2d_bytes));
+    CK(ws.mailbox());
+    // the scene's tables, unless the buffers hold them from the last run
+    if (ws.scene_version != hs.version || hs.version == 0) {
+        ws.scene_version = 0;
+        CK(upload(d_elems, hs.elems, st, out.h2d_bytes));
+        CK(upload(ws.elem_sphere, hs.elem_sphere, st, out.h2d_bytes));
+        CK(upload(ws.stage_cells, hs.stage_cells, st, out.h2d_bytes));
+        CK(upload(ws.grid_sphere, hs.grid_sphere, st, out.h2d_bytes));
+        CK(upload(ws.grid_elem, hs.grid_elem, st, out.h2d_bytes));
+        CK(upload(ws.beam_axis, hs.beam_axis, st, out.h2d_bytes));
+        CK(upload(ws.beam_range, hs.beam_range, st, out.h2d_bytes));
+        CK(upload(ws.beam_elem, hs.beam_elem, st, out.h2d_bytes));
+        CK(upload(d_optics, hs.optics, st, out.h2d_bytes));
+        CK(upload(d_surf, hs.surf_data, st, out.h2d_bytes));
+        CK(upload(d_tables, hs.tables, st, out.h2d_bytes));
+        CK(upload(d_bvh, hs.bvh, st, out.h2d_bytes));
+        CK(upload(d_bvh_items, hs.bvh_items, st, out.h2d_bytes));
+        CK(upload(d_cell_start, hs.cell_start, st, out.h2d_bytes));
+        CK(upload(d_cell_disc, hs.cell_disc, st, out.h2d_bytes));
+        CK(upload(ws.cell_par, hs.cell_par, st, out.h2d_bytes));
+        CK(upload(ws.cell_xa, hs.cell_xa, st, out.h2d_bytes));
+        CK(upload(ws.cell_xb, hs.cell_xb, st, out.h2d_bytes));
+        CK(upload(ws.cell_xc, hs.cell_xc, st, out.h2d_bytes));
+        CK(upload(ws.occ, hs.occ, st, out.h2d_bytes));
+        CK(upload(d_inv_cdf, hs.inv_cdf, st, out.h2d_bytes));
+        ws.scene_version = hs.version;
+    }
+    const uint64_t n_explicit = rq.n_explicit;
+    CK(d_expos.ensure(std::max<size_t>(n_explicit * 24, 16)));
+    CK(d_excos.ensure(std::max<size_t>(n_explicit * 24, 16)));
+    if (n_explicit) {
+        CK(cudaMemcpyAsync(d_expos.p, rq.ex_pos, n_explicit * 24, cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(d_excos.p, rq.ex_cos, n_explicit * 24, cudaMemcpyHostToDevice, st));
+        out.h2d_bytes += n_explicit * 48;
+    }
 
     SceneDev S = hs.dev;
     S.elems = d_elems.as<ElemRec>();
@@ -443,8 +474,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     S.sun.inv_cdf = hs.inv_cdf.empty() ? nullptr : d_inv_cdf.as<double>();
     S.seed = rq.seed;
     S.precision = rq.precision;
-    const bool explicit_mode = !rq.ex_pos.empty();
-    const uint64_t n_explicit = rq.ex_pos.size() / 3;
+    const bool explicit_mode = n_explicit > 0;
     S.explicit_rays = explicit_mode ? 1 : 0;
     S.ex_pos = d_expos.as<double>();
     S.ex_cos = d_excos.as<double>();
@@ -496,7 +526,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     CK(d_etotal.ensure(8));
     unsigned long long rec_cap = 0, save_cap = 0;
     (void)dev_sms;
-    CK(cudaStreamSynchronize(st));
     out.setup_ms = ms_since(t_setup);
 
     // room for `need` records in the run's record buffer, keeping the first `keep`
@@ -631,6 +660,28 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         cudaEvent_t t_first = new_event(), t_last = new_event();
         CK(cudaEventRecord(t_first, st));
         bool done = false;
+        // what the host reads after queued work -- run state, record count, counters and (small)
+        // accumulators -- in one wait; `fresh` until more work is queued
+        const bool acc_mailed = acc_n <= Workspace::kAccHost;
+        bool fresh = false;
+        auto read_back = [&]() -> cudaError_t {
+            cudaError_t e;
+            if ((e = cudaEventRecord(t_last, st)) ||
+                (e = cudaMemcpyAsync(&ws.mail->rs, drs, sizeof(RunState), cudaMemcpyDeviceToHost, st)) ||
+                (e = cudaMemcpyAsync(&ws.mail->ctr, d_ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st)))
+                return e;
+            out.d2h_bytes += sizeof(RunState) + sizeof(RunCounters);
+            if (rq.records) {
+                if ((e = cudaMemcpyAsync(&ws.mail->nrec, d_rec_count.p, 8, cudaMemcpyDeviceToHost, st))) return e;
+                out.d2h_bytes += 8;
+            }
+            if (acc_mailed && acc_n) {
+                if ((e = cudaMemcpyAsync(ws.acc_host, d_acc.p, acc_n * 8, cudaMemcpyDeviceToHost, st))) return e;
+                out.d2h_bytes += acc_n * 8;
+            }
+            fresh = true;
+            return cudaStreamSynchronize(st);
+        };
         if (rq.replay) {
             // saved stage data: the rays enter the second stage directly (no sun rays, no probe)
             const uint64_t n1 = rq.replay_rows.size() / 7;
@@ -659,9 +710,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             CK(cudaGetLastError());
             trace_ev.push_back({p1, p2});
             out.batches = 1;
-            unsigned long long nrec = 0;
-            if (rq.records) CK(cudaMemcpyAsync(&nrec, d_rec_count.p, 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
+            CK(read_back());
+            const unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
             if (rq.records && nrec > rec_cap) {
                 rec_cap = nrec + nrec / 4 + 4096;
                 continue;
@@ -806,12 +856,11 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 queued += n_all;
                 sun_next += n_all;
                 out.batches++;
+                fresh = false;
                 if (sync_each) {
-                    CK(cudaMemcpyAsync(&rs, drs, sizeof rs, cudaMemcpyDeviceToHost, st));
-                    out.d2h_bytes += sizeof rs;
-                    unsigned long long nrec = 0;
-                    if (rq.records) CK(cudaMemcpyAsync(&nrec, d_rec_count.p, 8, cudaMemcpyDeviceToHost, st));
-                    CK(cudaStreamSynchronize(st));
+                    CK(read_back());
+                    rs = ws.mail->rs;
+                    unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
                     const unsigned long long nrec_local = nrec;
                     bool overflow = rq.records && nrec > rec_cap;
                     if (multi) {  // a rank out of record room makes every rank re-run, in step
@@ -839,7 +888,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                     }
                     if (rq.records) {
                         nrec_run = nrec_local;
-                        out.d2h_bytes += 8;
                         if (!multi && rs.hits_done > 0)
                             rec_per_ray = std::max(1.0, 1.5 * double(nrec_run - n_pre) / double(rs.hits_done));
                     }
@@ -856,9 +904,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 if (multi && global_done == rq.n_hits) break;
             }
             if (restart) break;
-            CK(cudaMemcpyAsync(&rs, drs, sizeof rs, cudaMemcpyDeviceToHost, st));
-            out.d2h_bytes += sizeof rs;
-            CK(cudaStreamSynchronize(st));
+            if (!fresh) CK(read_back());
+            rs = ws.mail->rs;
             const uint64_t done_hits = multi ? global_done : rs.hits_done;
             if ((multi ? global_done == rq.n_hits : rs.reached != 0) || out.cancelled ||
                 (explicit_mode && sun_next >= n_explicit))
@@ -866,8 +913,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             if (!explicit_mode && sun_next > 0) p_est = std::max(double(done_hits) / double(sun_next), 1e-9);
         }
         if (restart) continue;
-        CK(cudaEventRecord(t_last, st));
-        CK(cudaStreamSynchronize(st));
+        if (!fresh) CK(read_back());  // no batch was needed
         float ms = 0;
         cudaEventElapsedTime(&ms, t_first, t_last);
         out.device_ms = ms;
@@ -887,14 +933,18 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             out.error = "run ended before the requested hits were numbered";
             return false;
         }
-        RunCounters c;
-        CK(cudaMemcpyAsync(&c, d_ctr.p, sizeof c, cudaMemcpyDeviceToHost, st));
+        RunCounters c = ws.mail->ctr;
         const auto tr = std::chrono::steady_clock::now();
-        std::vector<unsigned long long> accv(acc_n);
-        if (acc_n) CK(cudaMemcpyAsync(accv.data(), d_acc.p, acc_n * 8, cudaMemcpyDeviceToHost, st));
-        out.d2h_bytes += acc_n * 8 + sizeof c;
-        CK(cudaStreamSynchronize(st));
-        unsigned fe_fail = rq.precision ? take_fe_failures_mixed() : take_fe_failures_fp64();
+        std::vector<unsigned long long> accv;
+        if (acc_mailed) {
+            accv.assign(ws.acc_host, ws.acc_host + acc_n);
+        } else {
+            accv.resize(acc_n);
+            CK(cudaMemcpyAsync(accv.data(), d_acc.p, acc_n * 8, cudaMemcpyDeviceToHost, st));
+            out.d2h_bytes += acc_n * 8;
+            CK(cudaStreamSynchronize(st));
+        }
+        unsigned fe_fail = !hs.has_fe ? 0u : rq.precision ? take_fe_failures_mixed() : take_fe_failures_fp64();
         if (multi) {
             // the run's totals over all ranks: counts summed, SunRayCount (the cutting rank's;
             // the others' are below it), largest ray numbers and flags by max; integer, so exact
@@ -1133,6 +1183,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     if (!ws.stream) CK(cudaStreamCreateWithFlags(&ws.stream, cudaStreamNonBlocking));
     cudaStream_t st = ws.stream;
     uint64_t &h2d = out.h2d_bytes;
+    ws.scene_version = 0;  // the shared tables are copied over a single run's
     // the scene's shared tables
     CK(upload(ws.elems, hs.elems, st, h2d));
     CK(upload(ws.elem_sphere, hs.elem_sphere, st, h2d));
@@ -1482,7 +1533,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         for (size_t m = 0; m < rq.flux.size(); ++m)
             r.flux.emplace_back(a + flux_off[m], a + flux_off[m] + map_size(rq.flux[m]));
     }
-    if (rq.precision ? take_fe_failures_mixed() : take_fe_failures_fp64()) {
+    if (hs.has_fe && (rq.precision ? take_fe_failures_mixed() : take_fe_failures_fp64())) {
         out.error = "Interpolation failed to find nearby nodes to ray hit in FEA surface.";
         return false;
     }
