@@ -197,42 +197,46 @@ __device__ inline int aperture_in(const ElemRec &e, T x, T y, bool start_plane) 
 
 // ------------------------------------------------------------------------------------
 // Quadric closed forms: sphere, paraboloid, hyperboloid/ellipsoid, cylinder
-// (quadricsurfaceclosedform.cpp:58-308).  Returns 0 and (out, n, t) on success.
+// (quadricsurfaceclosedform.cpp:58-308), the solution and the normal apart so that a ray is
+// solved once and its hit completed from the path length.  The reference writes every term
+// with coefficients K and divisors a2, b2, c2; the ones that are 1 or 0 for a surface are left
+// out here, which changes no rounding (terms that were quotients are products with _rn
+// intrinsics, which mixed precision does not fuse into their sums).  Bound by the double pipe: a
+// cylinder's ten divisions by 1 and both solutions' divisions were most of its cost.
 // ------------------------------------------------------------------------------------
-__device__ inline int quadric_hit(const ElemRec &e, const double P[3], const double D[3], double out[3], double n[3],
-                           double &t) {
-    double zc = 0, kx = 1, ky = 1, kz = 1, a2 = 1, b2 = 1, c2 = 1, A, B, C;
+// path length t to the accepted solution; 0 on success
+__device__ inline int quadric_solve(const ElemRec &e, const double P[3], const double D[3], double &t) {
+    double A, B, C;
     const int s = e.surf | 0x20;
     const double xd = P[0], yd = P[1];
+    // K of the y terms: 0 for single-axis sections and cylinders
+    const bool ky = s == 'o' || (s != 't' && e.stype != kSurfSingleAxis);
     if (s == 'p') {
-        a2 = 2.0 / e.vcx;
-        b2 = e.vcy > 0.0 ? 2.0 / e.vcy : 1e10;
-        ky = (e.stype == kSurfSingleAxis) ? 0.0 : 1.0;
-        kz = 0.0;
-        A = D[0] * D[0] * kx / a2 + D[1] * D[1] * ky / b2;
-        B = 2.0 * (kx * xd * D[0] / a2 + ky * yd * D[1] / b2) - D[2] / c2;
-        C = kx * xd * xd / a2 + ky * yd * yd / b2 - P[2] / c2;
-    } else {
-        double rhs;
-        if (s == 's') {
-            ky = (e.stype == kSurfSingleAxis) ? 0.0 : 1.0;
-            const double r = 1.0 / e.vcx;
-            zc = r;
-            rhs = r * r;
-        } else if (s == 'o') {
-            kz = e.kappa;
-            zc = 1.0 / e.kappa / e.vcx;
-            rhs = 1.0 / e.kappa / (e.vcx * e.vcx);
-        } else {  // 't'
-            ky = 0.0;
-            const double r = 1.0 / e.curv_rev;
-            zc = r;
-            rhs = r * r;
+        const double a2 = e.q0, b2 = e.q1;
+        A = D[0] * D[0] / a2;
+        B = xd * D[0] / a2;
+        C = xd * xd / a2;
+        if (ky) {
+            A = A + D[1] * D[1] / b2;
+            B = B + yd * D[1] / b2;
+            C = C + yd * yd / b2;
         }
-        const double zd = P[2] - zc;
-        A = D[0] * D[0] * kx / a2 + D[1] * D[1] * ky / b2 + D[2] * D[2] * kz / c2;
-        B = 2.0 * (kx * xd * D[0] / a2 + ky * yd * D[1] / b2 + kz * zd * D[2] / c2);
-        C = kx * xd * xd / a2 + ky * yd * yd / b2 + kz * zd * zd / c2 - rhs;
+        B = 2.0 * B - D[2];
+        C = C - P[2];
+    } else {
+        const double kz = s == 'o' ? e.kappa : 1.0;
+        const double zd = P[2] - e.q0;
+        A = __dmul_rn(D[0], D[0]);
+        B = __dmul_rn(xd, D[0]);
+        C = __dmul_rn(xd, xd);
+        if (ky) {
+            A = __dadd_rn(A, __dmul_rn(D[1], D[1]));
+            B = __dadd_rn(B, __dmul_rn(yd, D[1]));
+            C = __dadd_rn(C, __dmul_rn(yd, yd));
+        }
+        A = A + D[2] * D[2] * kz;
+        B = 2.0 * (B + kz * zd * D[2]);
+        C = C + kz * zd * zd - e.q1;
     }
     if (fabs(A) < 1e-12) {
         const double t1 = -C / B;
@@ -240,44 +244,59 @@ __device__ inline int quadric_hit(const ElemRec &e, const double P[3], const dou
         t = t1;
     } else if (B * B > 4.0 * A * C) {
         const double q = sqrt(B * B - 4.0 * A * C);
-        const double t1 = (-B + q) / (2.0 * A);
         const double t2 = (-B - q) / (2.0 * A);
+        bool first = false;  // the other solution
         if (t2 > 0) {
             t = t2;
-            if (P[2] + t2 * D[2] > e.zap) t = t1;
+            first = P[2] + t2 * D[2] > e.zap;
+        } else if (t2 == 0 || t2 < 0) {
+            first = true;
+        } else {
+            return 1;
+        }
+        double t1 = 0.0;
+        if (first) {
+            t1 = (-B + q) / (2.0 * A);
+            if (t2 < 0 && !(t1 > 0)) return 1;
+            t = t1;
+        }
+        if (t2 > 0) {
             const bool finite_len = (s == 't') || (s == 's' && e.stype == kSurfSingleAxis);
             if (finite_len) {
                 const double yt = P[1] + t * D[1];
-                if (yt < -e.ap[2] / 2.0 || yt > e.ap[2] / 2.0) t = t1;
+                if (yt < -e.ap[2] / 2.0 || yt > e.ap[2] / 2.0) t = first ? t1 : (-B + q) / (2.0 * A);
             }
-        } else if (t2 == 0 || (t2 < 0 && t1 > 0)) {
-            t = t1;
-        } else {
-            return 1;
         }
     } else {
         return 1;
     }
-    out[0] = P[0] + t * D[0];
-    out[1] = P[1] + t * D[1];
-    out[2] = P[2] + t * D[2];
-    // the reference squares each gradient term as ((((2 K d)/a2) * 2) * K * d)/a2
-    const double gx = 2.0 * kx * out[0] / a2, gy = 2.0 * ky * out[1] / b2;
-    const double sx = (gx * 2.0 * kx * out[0]) / a2, sy = (gy * 2.0 * ky * out[1]) / b2;
+    return 0;
+}
+// the surface normal at out (the reference squares each gradient term as
+// ((((2 K d)/a2) * 2) * K * d)/a2)
+__device__ inline void quadric_normal(const ElemRec &e, const double out[3], double n[3]) {
+    const int s = e.surf | 0x20;
+    const bool ky = s == 'o' || (s != 't' && e.stype != kSurfSingleAxis);
     if (s == 'p') {
-        const double m = sqrt(sx + sy + 1.0);
+        const double a2 = e.q0, b2 = e.q1;
+        const double gx = 2.0 * out[0] / a2, gy = ky ? 2.0 * out[1] / b2 : 0.0 * out[1];
+        double m = (gx * 2.0 * out[0]) / a2;
+        if (ky) m = m + (gy * 2.0 * out[1]) / b2;
+        m = sqrt(m + 1.0);
         n[0] = -gx / m;
-        n[1] = -gy / m;
+        n[1] = ky ? -gy / m : -gy;
         n[2] = 1.0 / m;
     } else {
-        const double gz = 2.0 * kz * (out[2] - zc) / c2;
-        const double sz = (gz * 2.0 * kz * (out[2] - zc)) / c2;
-        const double m = sqrt(sx + sy + sz);
+        const double kz = s == 'o' ? e.kappa : 1.0, dz = out[2] - e.q0;
+        const double gx = 2.0 * out[0], gy = ky ? 2.0 * out[1] : 0.0 * out[1];
+        const double gz = 2.0 * kz * dz;
+        double m = __dmul_rn(gx * 2.0, out[0]);
+        if (ky) m = __dadd_rn(m, __dmul_rn(gy * 2.0, out[1]));
+        m = sqrt(m + gz * 2.0 * kz * dz);
         n[0] = -gx / m;
-        n[1] = -gy / m;
+        n[1] = ky ? -gy / m : -gy;
         n[2] = -gz / m;
     }
-    return 0;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1031,43 +1050,79 @@ static __device__ __noinline__ int cold_intersect(const SceneDev &S, const ElemR
     return newton_hit(e, S.surf_data, pe, ce, out, n, t);
 }
 
+// the ray in the element's frame, moved 1e-5 along itself
+__device__ __forceinline__ void element_ray(const ElemRec &e, const double ps[3], const double cs[3], double pe[3],
+                                            double ce[3]) {
+    to_local(e.R, e.o, ps, cs, pe, ce);
+    pe[0] = pe[0] + 1.0e-5 * ce[0];
+    pe[1] = pe[1] + 1.0e-5 * ce[1];
+    pe[2] = pe[2] + 1.0e-5 * ce[2];
+}
+// path length to a flat element's plane: the Newton iteration on z = 0 converges at its first
+// step (intersect.cpp:948-1007)
+__device__ __forceinline__ double flat_solve(const double pe[3], const double ce[3]) {
+    return (0.0 - pe[2] != 0.0) ? (0.0 - pe[2]) / (ce[2] + 0.00000000001) : 0.0;
+}
+__device__ __forceinline__ bool quadric_element(const ElemRec &e) {
+    return e.stype != kSurfFlat && closed_form_surface(e.stype, e.surf);
+}
+// the hit of a ray on a closed-form element at path length t: point, direction, normal (flipped
+// when hit from behind)
+__device__ __forceinline__ void complete_hit(const ElemRec &e, const double pe[3], const double ce[3],
+                                             const double out[3], double n[3], double t, Hit &h) {
+    const int back = (ce[0] * n[0] + ce[1] * n[1] + ce[2] * n[2] < 0) ? 0 : 1;
+    for (int q = 0; q < 3; ++q) {
+        h.pe[q] = out[q];
+        h.ce[q] = ce[q];
+        h.n[q] = back ? -n[q] : n[q];
+    }
+    h.plen = t;
+    h.back = back;
+}
+__device__ __forceinline__ void point_at(const ElemRec &e, const double pe[3], const double ce[3], double t,
+                                         double out[3]) {
+    out[0] = pe[0] + ce[0] * t;
+    out[1] = pe[1] + ce[1] * t;
+    out[2] = e.stype == kSurfFlat ? 0.0 : pe[2] + ce[2] * t;
+}
+// The hit on a closed-form element whose test (element_test) accepted the ray at path length t:
+// the same arithmetic without the solution and the aperture test.
+__device__ __forceinline__ void closed_hit_at(const ElemRec &e, const double ps[3], const double cs[3], double t, Hit &h) {
+    double pe[3], ce[3], out[3], n[3] = {0.0, 0.0, 1.0};
+    element_ray(e, ps, cs, pe, ce);
+    point_at(e, pe, ce, t, out);
+    if (e.stype != kSurfFlat) quadric_normal(e, out, n);
+    complete_hit(e, pe, ce, out, n, t, h);
+}
+
 // CLOSED: the element is known to have a closed-form surface (closed_form_surface), so the
 // out-of-line path is left out of the caller
 template <int MIXED, int CLOSED = 0>
 __device__ __forceinline__ bool element_test(const SceneDev &S, const ElemRec &e, const double ps[3],
                                              const double cs[3], double &plen, Hit *full) {
     double pe[3], ce[3];
-    to_local(e.R, e.o, ps, cs, pe, ce);
-    pe[0] = pe[0] + 1.0e-5 * ce[0];
-    pe[1] = pe[1] + 1.0e-5 * ce[1];
-    pe[2] = pe[2] + 1.0e-5 * ce[2];
+    element_ray(e, ps, cs, pe, ce);
     double out[3], n[3] = {0.0, 0.0, 1.0}, t = 0.0;
-    int err;
-    switch (e.stype) {
-        case kSurfFlat: {
-            // the Newton iteration on z = 0 converges at its first step (intersect.cpp:948-1007)
-            t = (0.0 - pe[2] != 0.0) ? (0.0 - pe[2]) / (ce[2] + 0.00000000001) : 0.0;
-            out[0] = pe[0] + ce[0] * t;
-            out[1] = pe[1] + ce[1] * t;
-            out[2] = 0.0;
-            err = 0;
-            break;
+    int err = 0;
+    const bool quadric = quadric_element(e);
+    if (e.stype == kSurfFlat) {
+        t = flat_solve(pe, ce);
+        point_at(e, pe, ce, t, out);
+    } else if (quadric) {
+        err = quadric_solve(e, pe, ce, t);
+        point_at(e, pe, ce, t, out);
+    } else if (CLOSED) {
+        return false;
+    } else {
+        // through copies: the out-of-line call takes addresses, which would keep the other
+        // surfaces' values in local memory too
+        double p2[3] = {pe[0], pe[1], pe[2]}, c2[3] = {ce[0], ce[1], ce[2]}, o2[3], n2[3] = {0.0, 0.0, 1.0}, t2 = 0.0;
+        err = cold_intersect(S, e, p2, c2, o2, n2, t2);
+        for (int q = 0; q < 3; ++q) {
+            out[q] = o2[q];
+            n[q] = n2[q];
         }
-        case kSurfCylinder:
-            err = quadric_hit(e, pe, ce, out, n, t);
-            break;
-        case kSurfTorus:
-            err = CLOSED ? 1 : cold_intersect(S, e, pe, ce, out, n, t);
-            break;
-        default: {
-            const int s = e.surf | 0x20;
-            const bool closed = (s == 'p') || (s == 's' && (e.stype == kSurfConic || e.stype == kSurfSingleAxis)) ||
-                                (s == 'o' && e.stype == kSurfConic);
-            if (closed)
-                err = quadric_hit(e, pe, ce, out, n, t);
-            else
-                err = CLOSED ? 1 : cold_intersect(S, e, pe, ce, out, n, t);
-        }
+        t = t2;
     }
     if (err > 0 || t < 0) return false;
     int in;
@@ -1080,14 +1135,8 @@ __device__ __forceinline__ bool element_test(const SceneDev &S, const ElemRec &e
     if (!(out[2] <= e.zap || s == 'm' || s == 'r')) return false;
     plen = t;
     if (full) {
-        const int back = (ce[0] * n[0] + ce[1] * n[1] + ce[2] * n[2] < 0) ? 0 : 1;
-        for (int q = 0; q < 3; ++q) {
-            full->pe[q] = out[q];
-            full->ce[q] = ce[q];
-            full->n[q] = back ? -n[q] : n[q];
-        }
-        full->plen = t;
-        full->back = back;
+        if (quadric) quadric_normal(e, out, n);
+        complete_hit(e, pe, ce, out, n, t, *full);
     }
     return true;
 }

@@ -1453,6 +1453,7 @@ bool flatten(Context *cx, HostScene &hs) {
             r.surf = e.surface;
             r.stype = e.stype;
             if (e.stype == kSurfFE) hs.has_fe = true;
+            quadric_constants(r);
             r.interaction = e.interaction;
             r.opt_front = e.optic_idx >= 0 ? 2 * e.optic_idx : -1;
             r.opt_back = e.optic_idx >= 0 ? 2 * e.optic_idx + 1 : -1;

@@ -22,7 +22,6 @@ static void resolve(const SceneDev &S, uint64_t s0, const ProbeOut &o, const Run
 }
 int launch_probe_fp64(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
                       cudaStream_t st) {
-    const uint32_t nb = (n + kProbeBlock - 1) / kProbeBlock;
     if (S.sun.grid_on && !S.explicit_rays && !S.sun.point_source) {
         if (launch_sun_probe_flat(S, s0, n, o, rs, st)) {
             int dev = 0, sms = 148;
@@ -39,7 +38,7 @@ int launch_probe_fp64(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut
             resolve<0>(S, s0, o, rs, st);
         return 2;
     }
-    k_probe<0><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs);
+    launch_k_probe<0>(S, s0, n, o, rs, st);
     return 1;
 }
 

@@ -91,7 +91,7 @@ struct Workspace {
     DevBuf hit_mask;  // one bit per sun ray of the batch, set for a hit
     DevBuf amb;       // mixed probe: count, then the rays left to the double-precision search
     // trace state and queues (one slot per hit-list entry of a batch)
-    DevBuf wf_sid, wf_raynum, wf_draw, wf_meta, wf_fe0, wf_p, wf_c, wf_q0, wf_q1, wf_qs, wf_counts;
+    DevBuf wf_sid, wf_raynum, wf_draw, wf_meta, wf_fe0, wf_p, wf_c, wf_t, wf_q0, wf_q1, wf_qs, wf_counts;
     DevBuf save_rows[2], save_count, replay_rows, replay_fe0;  // stage-data save / replay
     DevBuf ecount, ecursor, etotal, s_hits;  // the batch's hits sorted by first-stage element (HitRec)
     // record ordering: key counts / slots, scan partials, per-stage counts, merge runs, columns
@@ -121,15 +121,20 @@ struct Workspace {
     } *mail = nullptr;
     unsigned long long *acc_host = nullptr;  // the same for accumulators of up to kAccHost values
     static constexpr size_t kAccHost = 1u << 16;
-    cudaError_t mailbox() {
-        cudaError_t e = mail ? cudaSuccess : cudaMallocHost(&mail, sizeof(Mail));
-        if (e == cudaSuccess && !acc_host) e = cudaMallocHost(&acc_host, kAccHost * sizeof(unsigned long long));
+    cudaError_t mailbox() {  // one allocation: the accumulators' place follows the mail
+        if (mail) return cudaSuccess;
+        constexpr size_t kMail = (sizeof(Mail) + 63) / 64 * 64;
+        void *p = nullptr;
+        const cudaError_t e = cudaMallocHost(&p, kMail + kAccHost * sizeof(unsigned long long));
+        if (e == cudaSuccess) {
+            mail = static_cast<Mail *>(p);
+            acc_host = reinterpret_cast<unsigned long long *>(static_cast<char *>(p) + kMail);
+        }
         return e;
     }
     ~Workspace() {
         if (device >= 0) cudaSetDevice(device);
         if (mail) cudaFreeHost(mail);
-        if (acc_host) cudaFreeHost(acc_host);
         for (int k = 0; k < 2; ++k)
             if (pos_host[k]) cudaFreeHost(pos_host[k]);
         if (rec_host) {
@@ -191,7 +196,7 @@ static cudaError_t wf_buffers(Workspace &ws, const SceneDev &S, uint64_t cap, Wf
     const uint64_t nq = uint64_t(std::max(Q.n_queues, 1));
     if ((e = ws.wf_sid.ensure(cap * 8)) || (e = ws.wf_raynum.ensure(cap * 4)) || (e = ws.wf_draw.ensure(cap * 4)) ||
         (e = ws.wf_meta.ensure(cap * 16)) || (e = ws.wf_fe0.ensure(cap * 4)) || (e = ws.wf_p.ensure(cap * 24)) ||
-        (e = ws.wf_c.ensure(cap * 24)) || (e = ws.wf_q0.ensure(nq * cap * 4)) ||
+        (e = ws.wf_c.ensure(cap * 24)) || (e = ws.wf_t.ensure(cap * 8)) || (e = ws.wf_q0.ensure(nq * cap * 4)) ||
         (e = ws.wf_q1.ensure(nq * cap * 4)) || (e = ws.wf_qs.ensure(cap * 4)))
         return e;
     Q.rounds = 2 * nst;
@@ -208,6 +213,7 @@ static cudaError_t wf_buffers(Workspace &ws, const SceneDev &S, uint64_t cap, Wf
     W.fe0 = ws.wf_fe0.as<int>();
     W.p = ws.wf_p.as<double>();
     W.c = ws.wf_c.as<double>();
+    W.t = ws.wf_t.as<double>();
     W.cap = uint32_t(cap);
     return cudaSuccess;
 }

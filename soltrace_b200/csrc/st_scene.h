@@ -57,6 +57,7 @@ struct ElemRec {
     double kappa, vcx, vcy, curv_rev, cone_deg, ra, rs;
     double area;      // aperture area
     double bound_r;   // radius about the origin holding every accepted hit (<0: unbounded)
+    double q0, q1;    // quadric constants (quadric_constants): 'p' 2/Cx, 2/Cy; others centre z, right-hand side
     int shape;        // aperture code (lower-case char)
     int surf;         // surface code as given (char, case preserved)
     int stype;        // SurfType
@@ -67,6 +68,27 @@ struct ElemRec {
     int spl_n;        // spline points (x, y, y2 consecutive blocks)
     int pad_;
 };
+
+// The constants of an element's quadric (quadricsurfaceclosedform.cpp:91-173), each expression as
+// the reference evaluates it per ray.
+inline void quadric_constants(ElemRec &e) {
+    const int s = e.surf | 0x20;
+    if (s == 'p') {
+        e.q0 = 2.0 / e.vcx;
+        e.q1 = e.vcy > 0.0 ? 2.0 / e.vcy : 1e10;
+    } else if (s == 's') {
+        const double r = 1.0 / e.vcx;
+        e.q0 = r;
+        e.q1 = r * r;
+    } else if (s == 'o') {
+        e.q0 = 1.0 / e.kappa / e.vcx;
+        e.q1 = 1.0 / e.kappa / (e.vcx * e.vcx);
+    } else {
+        const double r = 1.0 / e.curv_rev;
+        e.q0 = r;
+        e.q1 = r * r;
+    }
+}
 
 struct OpticRec {
     double refl, trans, slope, spec;  // slope/spec in mrad

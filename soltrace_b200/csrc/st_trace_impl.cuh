@@ -70,9 +70,10 @@ __device__ __forceinline__ bool elem_hit(const SceneDev &S, const ElemRec &e, co
 }
 
 template <int MIXED, int ET = 0>
-__device__ inline int nearest_brute(const SceneDev &S, const StageRec &st, const double ps[3], const double cs[3]) {
+__device__ inline int nearest_brute(const SceneDev &S, const StageRec &st, const double ps[3], const double cs[3],
+                                    double &bp) {
     int best = -1;
-    double bp = 1e99;
+    bp = 1e99;
     for (int j = 0; j < st.n_elem; ++j) {
         const ElemRec &e = S.elems[st.first_elem + j];
         if (!e.enabled) continue;
@@ -90,7 +91,7 @@ __device__ inline int nearest_brute(const SceneDev &S, const StageRec &st, const
 // the float box arithmetic).
 template <int MIXED, int ET = 0>
 __device__ inline int nearest_bvh(const SceneDev &S, const StageRec &st, const double ps[3], const double cs[3],
-                                  int from) {
+                                  int from, double &bp) {
     const BvhNode *nodes = S.bvh + st.bvh_off;
     const int *items = S.bvh_items + st.bvh_items_off;
     const float ox = float(ps[0]), oy = float(ps[1]), oz = float(ps[2]);
@@ -103,7 +104,7 @@ __device__ inline int nearest_bvh(const SceneDev &S, const StageRec &st, const d
     int sp = 0;
     stack[sp++] = 0;
     int best = -1;
-    double bp = 1e99;
+    bp = 1e99;
     while (sp > 0) {
         const BvhNode nd = nodes[stack[--sp]];
         float t0x = (nd.lo[0] - ox) * ix, t1x = (nd.hi[0] - ox) * ix;
@@ -156,7 +157,7 @@ __device__ inline int nearest_bvh(const SceneDev &S, const StageRec &st, const d
 // ties), so the result is the brute-force search's.
 template <int MIXED, int ET = 0>
 __device__ inline int nearest_grid(const SceneDev &S, const StageRec &st, const double ps[3], const double cs[3],
-                                   int from) {
+                                   int from, double &bp) {
     const float ox = float(ps[0]), oy = float(ps[1]), oz = float(ps[2]);
     const float dx = float(cs[0]), dy = float(cs[1]), dz = float(cs[2]);
     // a ray leaving a flat element within its outgoing beam: that element's list stands in
@@ -199,7 +200,7 @@ __device__ inline int nearest_grid(const SceneDev &S, const StageRec &st, const 
     const int2 *cells = S.stage_cells + st.gcell_off;
     const float pad_o = 2e-6f * (fabsf(ox) + fabsf(oy) + fabsf(oz));
     int best = -1;
-    double bp = 1e99;
+    bp = 1e99;
     // the candidate list lives in shared memory, [slot][thread] (blocks have at most 256
     // threads), so that it neither takes registers nor goes to local memory
     constexpr int kCand = 8;
@@ -260,21 +261,16 @@ __device__ inline int nearest_grid(const SceneDev &S, const StageRec &st, const 
     return best;
 }
 
-template <int MIXED>
-__device__ __forceinline__ int nearest(const SceneDev &S, const StageRec &st, const double ps[3], const double cs[3],
-                                       int from = -1) {
-    if (st.grid_on) return nearest_grid<MIXED>(S, st, ps, cs, from);
-    return (st.bvh_off >= 0) ? nearest_bvh<MIXED>(S, st, ps, cs, from) : nearest_brute<MIXED>(S, st, ps, cs);
-}
-
-// nearest element with the code of search kind KIND only (stage_search_kind, st_launch.h)
+// Nearest element of a stage with the code of search kind KIND only (stage_search_kind,
+// st_launch.h; 0 holds every case), bp the path length to it.
 template <int MIXED, int KIND>
 __device__ __forceinline__ int nearest_kind(const SceneDev &S, const StageRec &st, const double ps[3],
-                                            const double cs[3], int from) {
+                                            const double cs[3], int from, double &bp) {
     constexpr int ET = (KIND & kSearchFlat) ? kEtFlat : (KIND & kSearchClosed) ? kEtClosed : 0;
-    if (KIND & kSearchBrute) return nearest_brute<MIXED, ET>(S, st, ps, cs);
-    if (st.grid_on) return nearest_grid<MIXED, ET>(S, st, ps, cs, from);
-    return (st.bvh_off >= 0) ? nearest_bvh<MIXED, ET>(S, st, ps, cs, from) : nearest_brute<MIXED, ET>(S, st, ps, cs);
+    if (KIND & kSearchBrute) return nearest_brute<MIXED, ET>(S, st, ps, cs, bp);
+    if (st.grid_on) return nearest_grid<MIXED, ET>(S, st, ps, cs, from, bp);
+    return (st.bvh_off >= 0) ? nearest_bvh<MIXED, ET>(S, st, ps, cs, from, bp)
+                             : nearest_brute<MIXED, ET>(S, st, ps, cs, bp);
 }
 
 // first test of a first-stage sun ray through the sun-plane grid (cells list the
@@ -289,6 +285,31 @@ __device__ __forceinline__ void sun_ray_in_stage(const SceneDev &S, double xs, d
     to_ref(sun.Rsun, sun.pos_sun_stage, psun, csun, pst, cst);
     to_ref(st.R, st.o, pst, cst, pg, cg);
     to_local(st.R, st.o, pg, cg, ps, cs);
+}
+// Every sun ray of a run has the same direction: one thread of a block computes it for all
+// (sun_dir, shared memory, then a barrier), and a ray computes its position alone.
+__device__ __forceinline__ void sun_dir_in_stage(const SceneDev &S, double cs[3]) {
+    double ps[3];
+    sun_ray_in_stage(S, S.sun.xmin, S.sun.ymin, ps, cs);
+}
+__device__ __forceinline__ void sun_pos_in_stage(const SceneDev &S, double xs, double ys, double ps[3]) {
+    double cs[3];
+    sun_ray_in_stage(S, xs, ys, ps, cs);  // the direction is left out as unused
+}
+// first-stage ray of stream index sid in stage coordinates: explicit, point source or sun ray
+// (direction sun_dir)
+__device__ __forceinline__ void first_stage_ray(const SceneDev &S, uint64_t sid, RayRng &rng, const double *sun_dir,
+                                                double ps[3], double cs[3]) {
+    if (!S.explicit_rays && !S.sun.point_source) {
+        const double xs = S.sun.xmin + (S.sun.xmax - S.sun.xmin) * rng.u();
+        const double ys = S.sun.ymin + (S.sun.ymax - S.sun.ymin) * rng.u();
+        sun_pos_in_stage(S, xs, ys, ps);
+        for (int q = 0; q < 3; ++q) cs[q] = sun_dir[q];
+        return;
+    }
+    double pg[3], cg[3], xs, ys;
+    make_ray(S, sid, rng, pg, cg, xs, ys);
+    to_local(S.stages[0].R, S.stages[0].o, pg, cg, ps, cs);
 }
 
 // Float pre-test of sun-plane point (fx, fy) against grid entry k: inside the padded disc
@@ -599,7 +620,12 @@ __device__ inline void bin_flux(const SceneDev &S, int si, int ej, bool absorbed
 // ------------------------------------------------------------------------------------
 // kernels
 // ------------------------------------------------------------------------------------
-template <int MIXED>
+// Probe of a first stage without a sun-plane grid, and of explicit and point-source rays: one
+// thread per ray, the search of the stage's kind only.  Bound by the double pipe and instruction
+// issue; KIND leaves out the other surfaces' code with its stack (the out-of-line call put every
+// ray's vectors in local memory) and the direction is computed once a block: the trough's 29.6e6
+// sun rays fell from 1.67 to 0.64 ms (with quadric_solve's fewer divisions).
+template <int MIXED, int KIND>
 __global__ void __launch_bounds__(kProbeBlock) k_probe(const __grid_constant__ SceneDev S, uint64_t s0, uint32_t n,
                                                         ProbeOut o, const RunState *rs) {
     const uint32_t i = blockIdx.x * kProbeBlock + threadIdx.x;
@@ -610,17 +636,15 @@ __global__ void __launch_bounds__(kProbeBlock) k_probe(const __grid_constant__ S
         if (threadIdx.x == 0) o.block_counts[blockIdx.x] = 0;
         return;
     }
+    __shared__ double sun_dir[3];
+    if (threadIdx.x == 0) sun_dir_in_stage(S, sun_dir);
+    __syncthreads();
     if (i < n) {
         RayRng rng;
         rng.init(S.seed, s0 + i, 0);
-        double pg[3], cg[3], xs, ys;
-        make_ray(S, s0 + i, rng, pg, cg, xs, ys);
-        const StageRec &st = S.stages[0];
-        double ps[3], cs[3];
-        to_local(st.R, st.o, pg, cg, ps, cs);
-        (void)xs;
-        (void)ys;
-        const int b = nearest<MIXED>(S, st, ps, cs);
+        double ps[3], cs[3], t;
+        first_stage_ray(S, s0 + i, rng, sun_dir, ps, cs);
+        const int b = nearest_kind<MIXED, KIND>(S, S.stages[0], ps, cs, -1, t);
         h = (b >= 0) ? uint32_t(b + 1) : 0u;
         if (o.hit_elem) o.hit_elem[i] = h;
         if (o.cand_el) {  // the list is every ray of the batch
@@ -632,6 +656,19 @@ __global__ void __launch_bounds__(kProbeBlock) k_probe(const __grid_constant__ S
     if (o.hit_mask && (threadIdx.x & 31) == 0) o.hit_mask[i / 32] = bal;
     const int c = __syncthreads_count(h != 0);
     if (threadIdx.x == 0) o.block_counts[blockIdx.x] = uint32_t(c);
+}
+template <int MIXED>
+static void launch_k_probe(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
+                           cudaStream_t st) {
+    const uint32_t nb = (n + kProbeBlock - 1) / kProbeBlock;
+    switch (stage_search_kind(S.stages[0])) {
+        case 6: k_probe<MIXED, 6><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs); break;
+        case 4: k_probe<MIXED, 4><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs); break;
+        case 3: k_probe<MIXED, 3><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs); break;
+        case 1: k_probe<MIXED, 1><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs); break;
+        case 2: k_probe<MIXED, 2><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs); break;
+        default: k_probe<MIXED, 0><<<nb, kProbeBlock, 0, st>>>(S, s0, n, o, rs);
+    }
 }
 
 // Probe of generated sun rays on a first stage culled by the sun-plane grid, in two
@@ -1336,6 +1373,7 @@ struct WfRay {
     uint32_t raynum, draw;
     int si, hits, last_j, next_j, fe0;
     double p[3], c[3];  // global while hits == 0 in stage si, stage coordinates after
+    double t;           // path length to element next_j
     bool moved;         // p, c changed since loaded
 };
 
@@ -1379,6 +1417,7 @@ __device__ __forceinline__ void wf_count_record(WfBlockCtr &c) {
     if ((threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&c.intersections, (unsigned long long)__popc(mask));
 }
 
+template <int MIXED>
 __device__ __forceinline__ WfRay wf_load(const WfState &W, uint32_t i) {
     WfRay r;
     r.sid = W.sid[i];
@@ -1390,6 +1429,7 @@ __device__ __forceinline__ WfRay wf_load(const WfState &W, uint32_t i) {
     r.last_j = m.z;
     r.next_j = m.w;
     r.fe0 = W.fe0[i];
+    if (!MIXED && r.next_j >= 0) r.t = W.t[i];
     for (int q = 0; q < 3; ++q) {
         r.p[q] = W.p[size_t(q) * W.cap + i];
         r.c[q] = W.c[size_t(q) * W.cap + i];
@@ -1398,6 +1438,7 @@ __device__ __forceinline__ WfRay wf_load(const WfState &W, uint32_t i) {
     return r;
 }
 
+template <int MIXED>
 __device__ __forceinline__ void wf_store(const WfState &W, uint32_t i, const WfRay &r, bool all) {
     if (all) {
         W.sid[i] = r.sid;
@@ -1406,6 +1447,7 @@ __device__ __forceinline__ void wf_store(const WfState &W, uint32_t i, const WfR
     W.draw[i] = r.draw;
     W.meta[i] = make_int4(r.si, r.hits, r.last_j, r.next_j);
     W.fe0[i] = r.fe0;
+    if (!MIXED && r.next_j >= 0) W.t[i] = r.t;  // read by kHitAt only
     if (all || r.moved)
         for (int q = 0; q < 3; ++q) {
             W.p[size_t(q) * W.cap + i] = r.p[q];
@@ -1542,7 +1584,7 @@ template <int MIXED, int RECORDS, int KIND = 0>
 __device__ __forceinline__ int wf_search(const SceneDev &S, const TraceOut &O, WfBlockCtr &c, WfRay &r) {
     double ps[3], cs[3];
     wf_stage_ray(S, r, ps, cs);
-    const int j = nearest_kind<MIXED, KIND>(S, S.stages[r.si], ps, cs, r.last_j);
+    const int j = nearest_kind<MIXED, KIND>(S, S.stages[r.si], ps, cs, r.last_j, r.t);
     if (j < 0) return wf_exit_stage<RECORDS>(S, O, c, r, ps, cs);
     r.next_j = j;
     return kWfShade;
@@ -1552,23 +1594,39 @@ template <int MIXED, int RECORDS>
 __device__ __forceinline__ int wf_shade_hit(const SceneDev &S, const TraceOut &O, WfBlockCtr &c, WfRay &r,
                                             const ElemRec &e, int j, const Hit &h);
 
-// shade step: the hit on element next_j and what the ray does there (raytrace.cpp:830-1000);
-// FLAT: the stage holds flat elements only; CLOSED: closed-form surfaces only
-template <int MIXED, int RECORDS, int FLAT = 0, int CLOSED = 0>
-__device__ __forceinline__ int wf_shade(const SceneDev &S, const TraceOut &O, WfBlockCtr &c, WfRay &r) {
-    const int si = r.si;
-    const StageRec &st = S.stages[si];
-    double ps[3], cs[3];
-    wf_stage_ray(S, r, ps, cs);
+// Shade step: the hit on element next_j and what the ray does there (raytrace.cpp:830-1000).
+// The hit is completed with the code of MODE: kHitAny any surface, kHitFlat a flat element,
+// kHitClosed a closed-form surface, each tested anew (the same arithmetic as the search);
+// kHitAt a closed-form surface at the path length the search found (r.t), without solving it
+// again.  Mixed precision tests anew: its fused multiply-adds need not round alike in the two
+// kernels, and a ray whose hit the second test rejects (about one in 1e8, z within rounding of
+// ZAperture) leaves the stage.
+constexpr int kHitAny = 0, kHitFlat = 1, kHitClosed = 2, kHitAt = 3;
+template <int MIXED, int CLOSED>
+constexpr int kShadeMode = !CLOSED ? kHitAny : MIXED ? kHitClosed : kHitAt;
+template <int MIXED, int RECORDS, int MODE>
+__device__ __forceinline__ int wf_shade_ray(const SceneDev &S, const TraceOut &O, WfBlockCtr &c, WfRay &r,
+                                            const double ps[3], const double cs[3]) {
+    const StageRec &st = S.stages[r.si];
     const int j = r.next_j;
     r.next_j = -1;
     const ElemRec &e = S.elems[st.first_elem + j];
     Hit h;
     double pl;
-    // re-test the chosen element for the full hit (same arithmetic as the search)
-    const bool hit = FLAT ? element_test_flat<MIXED>(e, ps, cs, pl, &h) : element_test<MIXED, CLOSED>(S, e, ps, cs, pl, &h);
-    if (!hit) return wf_exit_stage<RECORDS>(S, O, c, r, ps, cs);
+    if (MODE == kHitAt) {
+        closed_hit_at(e, ps, cs, r.t, h);
+    } else {
+        const bool hit = MODE == kHitFlat ? element_test_flat<MIXED>(e, ps, cs, pl, &h)
+                                          : element_test<MIXED, MODE == kHitClosed ? 1 : 0>(S, e, ps, cs, pl, &h);
+        if (!hit) return wf_exit_stage<RECORDS>(S, O, c, r, ps, cs);
+    }
     return wf_shade_hit<MIXED, RECORDS>(S, O, c, r, e, j, h);
+}
+template <int MIXED, int RECORDS, int MODE>
+__device__ __forceinline__ int wf_shade(const SceneDev &S, const TraceOut &O, WfBlockCtr &c, WfRay &r) {
+    double ps[3], cs[3];
+    wf_stage_ray(S, r, ps, cs);
+    return wf_shade_ray<MIXED, RECORDS, MODE>(S, O, c, r, ps, cs);
 }
 
 // the hit h of the ray on element j of its stage and what the ray does there
@@ -1679,14 +1737,18 @@ __device__ __forceinline__ int wf_shade_hit(const SceneDev &S, const TraceOut &O
 // stage and are shaded on the element the probe found.
 // FLAT 1: the first stage holds flat elements only; 2: besides, its search kind is
 // kSearchFlat, and the rays it reflects are searched for blocking in this kernel (their
-// results go to round 0's shade queue and to the search queue of the ray's stage).
+// results go to round 0's shade queue and to the search queue of the ray's stage); 3: its
+// surfaces are all closed-form.
 template <int MIXED, int RECORDS, int FLAT>
-__global__ void __launch_bounds__(kTraceBlock, FLAT ? (MIXED ? kWfFirstFlatMinBlocksMixed : kWfFirstFlatMinBlocks)
-                                                    : kWfShadeMinBlocks) k_wf_first(
+__global__ void __launch_bounds__(kTraceBlock, FLAT == 3 ? kWfFirstClosedMinBlocks
+                                               : FLAT    ? (MIXED ? kWfFirstFlatMinBlocksMixed : kWfFirstFlatMinBlocks)
+                                                         : kWfShadeMinBlocks) k_wf_first(
     const __grid_constant__ SceneDev S, const HitRec *hits, const uint32_t *total,
     const RunState *rs, TraceOut O, WfState W, const __grid_constant__ WfQueues Q) {
     __shared__ WfBlockCtr c;
     __shared__ WfPushSh psh;
+    __shared__ double sun_dir[3];
+    if (threadIdx.x == 0) sun_dir_in_stage(S, sun_dir);
     wf_push_init(psh);
     wf_ctr_init(c);
     uint32_t n = 0, take = 0, raynum_base = 0;
@@ -1702,6 +1764,7 @@ __global__ void __launch_bounds__(kTraceBlock, FLAT ? (MIXED ? kWfFirstFlatMinBl
     for (uint32_t i = blockIdx.x * kTraceBlock + threadIdx.x; i < n_round; i += stride) {
         bool live = false;
         WfRay r;
+        double ps[3], cs[3];
         if (i < n) {
             const HitRec hr = hits[i];
             live = hr.rank < take;
@@ -1710,8 +1773,7 @@ __global__ void __launch_bounds__(kTraceBlock, FLAT ? (MIXED ? kWfFirstFlatMinBl
                 r.raynum = raynum_base + hr.rank + 1;
                 RayRng rng;
                 rng.init(S.seed, r.sid, 0);
-                double xs, ys;
-                make_ray(S, r.sid, rng, r.p, r.c, xs, ys);
+                first_stage_ray(S, r.sid, rng, sun_dir, ps, cs);
                 r.draw = rng.k;
                 r.si = 0;
                 r.hits = 0;
@@ -1724,12 +1786,12 @@ __global__ void __launch_bounds__(kTraceBlock, FLAT ? (MIXED ? kWfFirstFlatMinBl
         int kb = -1, status = kWfDone;
         if (live) {
             wf_stage_enter(c, 0, r.raynum);
-            // (an entry without a known element is searched in the first round)
-            status = (r.next_j >= 0) ? wf_shade<MIXED, RECORDS, FLAT ? 1 : 0>(S, O, c, r) : int(kWfSearch);
+            constexpr int kMode = FLAT == 3 ? kHitClosed : FLAT ? kHitFlat : kHitAny;
+            status = wf_shade_ray<MIXED, RECORDS, kMode>(S, O, c, r, ps, cs);
             // FLAT 2: the ray still in the first stage is searched here (its blocking search)
             if (FLAT == 2 && status == kWfSearch && r.si == 0) status = wf_search<MIXED, RECORDS, kSearchFlat>(S, O, c, r);
             if (status != kWfDone) {
-                wf_store(W, i, r, true);
+                wf_store<MIXED>(W, i, r, true);
                 if (status == kWfSearch) kb = Q.stage_queue[r.si];
             }
         }
@@ -1770,7 +1832,7 @@ __global__ void __launch_bounds__(kTraceBlock, kWfShadeMinBlocks) k_wf_replay(
             r.fe0 = in.fe0 ? in.fe0[i] : -1;
             r.moved = true;
             wf_stage_enter(c, 1, r.raynum);
-            wf_store(W, i, r, true);
+            wf_store<MIXED>(W, i, r, true);
         }
         wf_block_push(psh, nullptr, nullptr, false, Q.search[0], Q.cap, Q.counts, live ? int(Q.stage_queue[1]) : -1,
                       i);
@@ -1805,9 +1867,9 @@ __global__ void __launch_bounds__(kTraceBlock, SearchBounds<KIND>::min_blocks) k
         uint32_t i = 0;
         if (q < n) {
             i = q_in[q];
-            WfRay ray = wf_load(W, i);
+            WfRay ray = wf_load<MIXED>(W, i);
             status = wf_search<MIXED, RECORDS, KIND>(S, O, c, ray);
-            if (status != kWfDone) wf_store(W, i, ray, false);
+            if (status != kWfDone) wf_store<MIXED>(W, i, ray, false);
             if (status == kWfSearch) kb = Q.stage_queue[ray.si];
         }
         wf_block_push(psh, Q.shade, cnt + nq, status == kWfShade, Q.search[(r + 1) & 1], Q.cap, cnt + nq + 1, kb, i);
@@ -1836,10 +1898,10 @@ __global__ void __launch_bounds__(kTraceBlock, CLOSED ? (MIXED ? kWfClosedShadeM
         uint32_t i = 0;
         if (q < n) {
             i = Q.shade[q];
-            WfRay ray = wf_load(W, i);
-            const int status = wf_shade<MIXED, RECORDS, 0, CLOSED>(S, O, c, ray);
+            WfRay ray = wf_load<MIXED>(W, i);
+            const int status = wf_shade<MIXED, RECORDS, kShadeMode<MIXED, CLOSED>>(S, O, c, ray);
             if (status != kWfDone) {
-                wf_store(W, i, ray, false);
+                wf_store<MIXED>(W, i, ray, false);
                 kb = Q.stage_queue[ray.si];
             }
         }
@@ -1863,10 +1925,10 @@ __global__ void __launch_bounds__(kTraceBlock, kWfShadeMinBlocks) k_wf_finish(co
         const uint32_t n = cnt[k];
         const uint32_t *q_in = k < nq ? Q.search[R & 1] + size_t(k) * Q.cap : Q.shade;
         for (uint32_t q = blockIdx.x * kTraceBlock + threadIdx.x; q < n; q += gridDim.x * kTraceBlock) {
-            WfRay r = wf_load(W, q_in[q]);
+            WfRay r = wf_load<MIXED>(W, q_in[q]);
             int status = (r.next_j >= 0) ? int(kWfShade) : int(kWfSearch);
             while (status != kWfDone)
-                status = (status == kWfShade) ? wf_shade<MIXED, RECORDS, 0, CLOSED>(S, O, c, r)
+                status = (status == kWfShade) ? wf_shade<MIXED, RECORDS, kShadeMode<MIXED, CLOSED>>(S, O, c, r)
                                               : wf_search<MIXED, RECORDS, CLOSED ? kSearchClosed : 0>(S, O, c, r);
         }
     }
@@ -1891,11 +1953,12 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
                      const uint32_t *total, const RunState *rs, const TraceOut &O, const WfState &W,
                      const WfQueues &Q, const ReplayIn *replay, cudaStream_t st) {
     // persistent grids: every block the kernels can keep resident on every SM
-    static int per_sm[7] = {0, 0, 0, 0, 0, 0, 0};
+    static int per_sm[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (per_sm[0] == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_wf_first<MIXED, RECORDS, 0>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[4], k_wf_first<MIXED, RECORDS, 1>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[5], k_wf_first<MIXED, RECORDS, 2>, kTraceBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[7], k_wf_first<MIXED, RECORDS, 3>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_wf_shade<MIXED, RECORDS, 0>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[3], k_wf_shade<MIXED, RECORDS, 1>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_wf_finish<MIXED, RECORDS, 0>, kTraceBlock, 0);
@@ -1917,6 +1980,9 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
                                                                                  O, W, Q);
     else if (S.stages[0].flat_only)  // a first stage of flat elements only
         k_wf_first<MIXED, RECORDS, 1><<<sms * per_sm[4], kTraceBlock, 0, st>>>(S, hits, total, rs,
+                                                                                 O, W, Q);
+    else if (S.stages[0].closed_only)
+        k_wf_first<MIXED, RECORDS, 3><<<sms * per_sm[7], kTraceBlock, 0, st>>>(S, hits, total, rs,
                                                                                  O, W, Q);
     else
         k_wf_first<MIXED, RECORDS, 0><<<sms * per_sm[0], kTraceBlock, 0, st>>>(S, hits, total, rs,
