@@ -134,8 +134,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 64 accumulator columns of the warp's 32 lanes in one load and one wait (the fused kernel's
-// epilogue: a wait per 16 columns would serialise sixteen tensor-memory round trips per layer)
+// 64 accumulator columns of the warp's 32 lanes in one load and one wait
 __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float v[64]) {
     uint32_t r[64];
     asm volatile(
@@ -156,6 +155,23 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float v[64]) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 accumulator columns of the warp's 32 lanes
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // Stage rows [r0, r0 + R) x K [k0, k0 + kBK) of an operand (element (r, k) at src[r lr + k lk],
@@ -711,26 +727,31 @@ __global__ void k_to_bf16(long long n, const float *x, __nv_bfloat16 *y) {
 // layer; the weights stream through a ring of shared-memory stages, each one bulk copy
 // (cp.async.bulk, completion counted on the stage's mbarrier) of a block that the packing
 // kernel already laid out in that layout.  Roles:
-//   warps 0-3 (epilogue): load the tile's inputs into X; per layer read the accumulator back
-//     (warp w owns tensor-memory lanes 32w..32w+31, thread = row), add the bias, ReLU, round
-//     to bf16 and write X for the next layer; on the output layer apply scale/clamp and write
-//     the rows or add them into their group's sums;
-//   warp 4, one thread (loader): issues the weight stages, kRing ahead of their use, across
+//   warps 0-7 (epilogue): load the tile's inputs into X; per layer read the accumulator back
+//     64 columns at a time (warp w owns tensor-memory lanes 32 (w % 4) .. + 31, thread = row,
+//     and half of the 64 columns), add the bias, ReLU, round to bf16 and write that slice of X for
+//     the next layer; on the output layer apply scale/clamp and write the rows or add them into
+//     their group's sums;
+//   warp 8, one thread (loader): issues the weight stages, kRing ahead of their use, across
 //     layers and tiles (the next layer's weights arrive while the epilogue runs);
-//   warp 5, one thread (MMA issuer): per layer waits for X, per stage for its weights, issues
-//     the tcgen05.mma (128 x 256 x 16 each) and commits the stage back to the loader; the
-//     accumulator's commit wakes the epilogue.
+//   warp 9, one thread (MMA issuer): per stage waits for its weights and for the 64-wide slice of
+//     X they multiply, issues the tcgen05.mma (128 x 256 x 16 each) and commits the stage back
+//     to the loader; the accumulator's commit wakes the epilogue.
 // Two accumulators (2 x 256 tensor-memory columns) alternate between units (a layer, or a
-// 256-wide chunk of the output layer), so an output chunk's epilogue overlaps the next
-// chunk's products.  Every wait is bounded; one that runs out sets the error flag and a shared
-// abort flag that ends every role's loop, and the CTA drains its own copies and products
-// before freeing tensor memory.
+// 256-wide chunk of the output layer), so a layer's products start on the first slice of X while
+// the epilogue still writes the others, and an output chunk's epilogue overlaps the next
+// chunk's products.  With four epilogue warps and one barrier for the whole of X the tensor
+// cores waited for the epilogue of every hidden layer: 64 x 2,000 rows of the 6-layer network
+// took 338 us there and take 221 here.  Every wait is bounded; one that runs out sets the error
+// flag and a shared abort flag that ends every role's loop, and the CTA drains its own copies and
+// products before freeing tensor memory.
 constexpr int kWidth = 256;                       // hidden width: the MMA N and the next layer's K
 constexpr int kRing = 4;                          // weight stages in flight
 constexpr int kStageBytes = kWidth * kBK * 2;     // 32 KB: a 256 x 64 weight block
 constexpr int kFirstBytes = kWidth * 16 * 2;      // 8 KB: the first layer's 256 x 16 block
 constexpr int kXBytes = kBM * kWidth * 2;         // 64 KB: a 128-row activation tile
-constexpr int kFusedThreads = 192;
+constexpr int kFusedThreads = 320;                // warps 0-7 epilogue, 8 loader, 9 products
+constexpr int kSlices = kWidth / kBK;             // 64-wide slices of X
 constexpr int kMaxLayers = 8;
 constexpr int kMaxOut = 4096;
 
@@ -767,13 +788,18 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *X = smem;
     unsigned char *ring = smem + kXBytes;
-    __shared__ __align__(8) uint64_t full[kRing], empty[kRing], acc_full[2], acc_free[2], x_ready, drain;
+    float *bias_sh = reinterpret_cast<float *>(ring + kRing * kStageBytes);  // every layer's, end to end
+    __shared__ __align__(8) uint64_t full[kRing], empty[kRing], acc_full[2], acc_free[2], x_ready[kSlices], drain;
     __shared__ uint32_t tmem_sh;
     __shared__ volatile int abort_flag;
     __shared__ unsigned issued_sh, consumed_sh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (g.M + kBM - 1) / kBM;
     const int L = g.n_layers, NC = g.n_out / kWidth;
+    for (int k = threadIdx.x; k < (L - 1) * kWidth + g.n_out; k += kFusedThreads) {
+        const int l = min(k / kWidth, L - 1);
+        bias_sh[k] = g.bias[l][k - l * kWidth];
+    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < kRing; ++i) {
             mbar_init(&full[i], 1);
@@ -781,9 +807,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_free[i], 128);
+            mbar_init(&acc_free[i], 256);
         }
-        mbar_init(&x_ready, 128);
+        for (int i = 0; i < kSlices; ++i) mbar_init(&x_ready[i], 256);
         mbar_init(&drain, 1);
         abort_flag = 0;
         issued_sh = consumed_sh = 0;
@@ -800,7 +826,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
     const uint32_t tmem = tmem_sh;
     const int S = stages_per_tile(L, g.n_out);
 
-    if (warp == 4) {
+    if (warp == 8) {
         // ---- loader ----
         if (lane == 0) {
             unsigned q = 0;
@@ -817,19 +843,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
             }
             issued_sh = q;
         }
-    } else if (warp == 5) {
+    } else if (warp == 9) {
         // ---- MMA issuer ----
         if (lane == 0) {
             constexpr uint32_t idesc = instr_desc(kWidth);
-            unsigned q = 0, u = 0, xr = 0;
+            unsigned q = 0, u = 0, x0 = 0, x1 = 0;  // x0, x1: phases of slice 0 (a layer each) and of the others
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
                 for (int l = 0; l < L && ok; ++l) {
-                    if (!mbar_wait_or_abort(&x_ready, xr & 1u, &abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    ++xr;
                     const int chunks = (l == L - 1) ? NC : 1;
                     const int nst = (l == 0) ? 1 : kWidth / kBK;
                     for (int c = 0; c < chunks && ok; ++c, ++u) {
@@ -841,7 +862,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         for (int s = 0; s < nst; ++s, ++q) {
                             const int slot = q % kRing;
-                            if (!mbar_wait_or_abort(&full[slot], (q / kRing) & 1u, &abort_flag)) {
+                            if (!mbar_wait_or_abort(&full[slot], (q / kRing) & 1u, &abort_flag) ||
+                                (c == 0 && !mbar_wait_or_abort(&x_ready[s], (s ? x1 : x0) & 1u, &abort_flag))) {
                                 ok = false;
                                 break;
                             }
@@ -860,6 +882,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                         }
                         if (ok) mma_commit(&acc_full[b]);
                     }
+                    ++x0;
+                    if (l > 0) ++x1;
                 }
             }
             if (!ok) abort_flag = 1;
@@ -869,32 +893,27 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
             mbar_wait(&drain, 0);
         }
     } else {
-        // ---- epilogue: warps 0-3, thread = row of the tile ----
-        const int r = threadIdx.x;
+        // ---- epilogue: warps 0-7, thread = row of the tile and half of every 64 columns ----
+        const int r = threadIdx.x & 127, half = warp >> 2;
         unsigned u = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
             const int row = t * kBM + r;
-            // inputs, zero-padded to K = 16 (two core-matrix columns)
+            // inputs, zero-padded to K = 16 (two core-matrix columns, one per half)
             {
-                unsigned short h[16];
+                unsigned short h[8];
 #pragma unroll
-                for (int e = 0; e < 16; ++e)
-                    h[e] = (row < g.M && e < g.d_in) ? __bfloat16_as_ushort(g.x[row * g.ldx + e]) : (unsigned short)0;
-#pragma unroll
-                for (int kc = 0; kc < 2; ++kc) {
-                    const uint4 v = make_uint4(h[8 * kc] | (uint32_t(h[8 * kc + 1]) << 16),
-                                               h[8 * kc + 2] | (uint32_t(h[8 * kc + 3]) << 16),
-                                               h[8 * kc + 4] | (uint32_t(h[8 * kc + 5]) << 16),
-                                               h[8 * kc + 6] | (uint32_t(h[8 * kc + 7]) << 16));
-                    *reinterpret_cast<uint4 *>(X + (kc * 16 + r / 8) * 128 + (r % 8) * 16) = v;
-                }
+                for (int e = 0; e < 8; ++e)
+                    h[e] = (row < g.M && 8 * half + e < g.d_in) ? __bfloat16_as_ushort(g.x[row * g.ldx + 8 * half + e])
+                                                                : (unsigned short)0;
+                *reinterpret_cast<uint4 *>(X + (half * 16 + r / 8) * 128 + (r % 8) * 16) =
+                    make_uint4(h[0] | (uint32_t(h[1]) << 16), h[2] | (uint32_t(h[3]) << 16),
+                               h[4] | (uint32_t(h[5]) << 16), h[6] | (uint32_t(h[7]) << 16));
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(&x_ready);
+            mbar_arrive(&x_ready[0]);
             for (int l = 0; l < L && ok; ++l) {
                 const int chunks = (l == L - 1) ? NC : 1;
-                const float *bias = g.bias[l];
                 for (int c = 0; c < chunks; ++c, ++u) {
                     const int b = u & 1;
                     // warp-uniform: the tensor-memory loads below are warp-collective
@@ -903,83 +922,92 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ta = tmem + (uint32_t(warp * 32) << 16) + uint32_t(b * kWidth);
+                    const uint32_t ta = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(b * kWidth);
+                    const float4 *bias = reinterpret_cast<const float4 *>(bias_sh + l * kWidth + c * kWidth);
                     if (l < L - 1) {
-                        for (int c64 = 0; c64 < kWidth; c64 += 64) {
-                            float w64[64];
-                            tmem_ld64(ta + uint32_t(c64), w64);
+                        for (int s = 0; s < kSlices; ++s) {
+                            const int c0 = s * kBK + half * 32;
+                            float v[32];
+                            tmem_ld32(ta + uint32_t(c0), v);
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const float *v = w64 + 16 * q;
-                                const int c0 = c64 + 16 * q;
-                                uint32_t p[8];
+                            for (int q = 0; q < 4; ++q) {  // a K chunk of eight columns each
+                                const float4 b0 = bias[c0 / 4 + 2 * q], b1 = bias[c0 / 4 + 2 * q + 1];
+                                const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                                uint32_t p[4];
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) {
-                                    const float a0 = fmaxf(v[2 * i] + __ldg(bias + c0 + 2 * i), 0.f);
-                                    const float a1 = fmaxf(v[2 * i + 1] + __ldg(bias + c0 + 2 * i + 1), 0.f);
+                                for (int i = 0; i < 4; ++i) {
+                                    const float a0 = fmaxf(v[8 * q + 2 * i] + bb[2 * i], 0.f);
+                                    const float a1 = fmaxf(v[8 * q + 2 * i + 1] + bb[2 * i + 1], 0.f);
                                     p[i] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(a0))) |
                                            (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(a1))) << 16);
                                 }
-                                const int kc = c0 / 8;
-                                *reinterpret_cast<uint4 *>(X + (kc * 16 + r / 8) * 128 + (r % 8) * 16) =
+                                *reinterpret_cast<uint4 *>(X + ((c0 / 8 + q) * 16 + r / 8) * 128 + (r % 8) * 16) =
                                     make_uint4(p[0], p[1], p[2], p[3]);
-                                *reinterpret_cast<uint4 *>(X + ((kc + 1) * 16 + r / 8) * 128 + (r % 8) * 16) =
-                                    make_uint4(p[4], p[5], p[6], p[7]);
                             }
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                            if (s + 1 == kSlices) {
+                                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                                mbar_arrive(&acc_free[b]);
+                            }
+                            mbar_arrive(&x_ready[s]);
                         }
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        mbar_arrive(&acc_free[b]);
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        mbar_arrive(&x_ready);
                     } else {
                         const int n0 = c * kWidth;
                         const bool valid = row < g.M;
                         const long long grp = (long long)(valid ? row : g.M - 1) / (g.mode == 1 ? g.group_rows : 1);
                         const long long grp0 = __shfl_sync(0xffffffffu, grp, 0);
                         const bool uniform = __all_sync(0xffffffffu, grp0 == grp) && g.mode == 1;
-                        for (int c64 = 0; c64 < kWidth; c64 += 64) {
-                          float w64[64];
-                          tmem_ld64(ta + uint32_t(c64), w64);
+                        for (int s = 0; s < kSlices; ++s) {
+                            float w32[32];
+                            tmem_ld32(ta + uint32_t(s * kBK + half * 32), w32);
 #pragma unroll
-                          for (int q = 0; q < 4; ++q) {
-                            float *v = w64 + 16 * q;
-                            const int c0 = c64 + 16 * q;
+                            for (int q = 0; q < 2; ++q) {
+                                float *v = w32 + 16 * q;
+                                const int c0 = s * kBK + half * 32 + 16 * q;
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                float y = (v[i] + __ldg(bias + n0 + c0 + i)) * g.scale;
-                                if (g.clamp) y = fmaxf(y, 0.f);
-                                v[i] = valid ? y : 0.f;
-                            }
-                            const int col = n0 + c0;
-                            if (g.mode == 0) {
-                                if (valid) {
-                                    float4 *o = reinterpret_cast<float4 *>(g.out + (long long)row * g.n_out + col);
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i)
-                                        o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                                for (int i = 0; i < 4; ++i) {
+                                    const float4 bb = bias[c0 / 4 + i];
+                                    v[4 * i] += bb.x;
+                                    v[4 * i + 1] += bb.y;
+                                    v[4 * i + 2] += bb.z;
+                                    v[4 * i + 3] += bb.w;
                                 }
-                            } else if (uniform) {
-                                // the warp's 32 rows share a group: halve the 16 columns' sums across
-                                // lanes (16 shuffles), then one atomic per column
 #pragma unroll
-                                for (int d = 16, w = 8; d >= 2; d >>= 1, w >>= 1) {
+                                for (int i = 0; i < 16; ++i) {
+                                    float y = v[i] * g.scale;
+                                    if (g.clamp) y = fmaxf(y, 0.f);
+                                    v[i] = valid ? y : 0.f;
+                                }
+                                const int col = n0 + c0;
+                                if (g.mode == 0) {
+                                    if (valid) {
+                                        float4 *o = reinterpret_cast<float4 *>(g.out + (long long)row * g.n_out + col);
 #pragma unroll
-                                    for (int i = 0; i < w; ++i) {
-                                        const bool hi = (lane & d) != 0;
-                                        const float send = hi ? v[i] : v[i + w];
-                                        const float keep = hi ? v[i + w] : v[i];
-                                        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+                                        for (int i = 0; i < 4; ++i)
+                                            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                                     }
-                                }
-                                v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                                const int k = ((lane & 16) ? 8 : 0) + ((lane & 8) ? 4 : 0) + ((lane & 4) ? 2 : 0) +
-                                              ((lane & 2) ? 1 : 0);
-                                if ((lane & 1) == 0) atomicAdd(g.out + grp * g.n_out + col + k, v[0]);
-                            } else if (valid) {
+                                } else if (uniform) {
+                                    // the warp's 32 rows share a group: halve the 16 columns' sums across
+                                    // lanes (16 shuffles), then one atomic per column
 #pragma unroll
-                                for (int i = 0; i < 16; ++i) atomicAdd(g.out + grp * g.n_out + col + i, v[i]);
+                                    for (int d = 16, w = 8; d >= 2; d >>= 1, w >>= 1) {
+#pragma unroll
+                                        for (int i = 0; i < w; ++i) {
+                                            const bool hi = (lane & d) != 0;
+                                            const float send = hi ? v[i] : v[i + w];
+                                            const float keep = hi ? v[i + w] : v[i];
+                                            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+                                        }
+                                    }
+                                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                                    const int k = ((lane & 16) ? 8 : 0) + ((lane & 8) ? 4 : 0) + ((lane & 4) ? 2 : 0) +
+                                                  ((lane & 2) ? 1 : 0);
+                                    if ((lane & 1) == 0) atomicAdd(g.out + grp * g.n_out + col + k, v[0]);
+                                } else if (valid) {
+#pragma unroll
+                                    for (int i = 0; i < 16; ++i) atomicAdd(g.out + grp * g.n_out + col + i, v[i]);
+                                }
                             }
-                          }
                         }
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         mbar_arrive(&acc_free[b]);
@@ -1158,7 +1186,8 @@ long long packed_elems(int n_layers, const int *dims) {
 }
 
 int launch_fused(const FusedArgs &a, cudaStream_t st) {
-    constexpr int smem = kXBytes + kRing * kStageBytes;
+    // X, the weight ring and the biases (at most 7 x 256 + 4096)
+    constexpr int smem = kXBytes + kRing * kStageBytes + ((kMaxLayers - 1) * kWidth + kMaxOut) * 4;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
     static int sms[64] = {0};
