@@ -1177,6 +1177,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
     hs.cell_xb.clear();
     hs.cell_xc.clear();
     hs.occ.clear();
+    hs.hit_rate = 0.0;
     if (!sun.point_source && st.elems.size() >= 4) {
         bool bounded = true;
         double rmax = 0;
@@ -1319,6 +1320,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
                     mulv(Rs, nz3, n2);
                     const double det = a2[0] * b2[1] - a2[1] * b2[0];
                     const double la = sqrt(sq(a2[0]) + sq(a2[1])), lb = sqrt(sq(b2[0]) + sq(b2[1]));
+                    if (!never(e)) hs.hit_rate += 4.0 * fabs(det) / (W * H);
                     ecx[j] = c2[0];
                     ecy[j] = c2[1];
                     xb[j] = float4{0.f, 0.f, 0.f, 0.f};
@@ -1342,6 +1344,7 @@ bool sun_setup(Context *cx, HostScene &hs) {
                 }
             }
             // (start, end) pair per cell: cell c at [2c, 2c + 1], read on the device as one int2
+            hs.hit_rate = std::min(hs.hit_rate, 1.0);
             hs.cell_start.assign(2 * size_t(nx) * ny, 0);
             int at = 0;
             for (size_t c = 0; c < cells.size(); ++c) {
@@ -1863,6 +1866,7 @@ bool build_position(const Context *cx, const HostScene &hs, const double sun_xyz
     out.cell_xb.swap(h.cell_xb);
     out.cell_xc.swap(h.cell_xc);
     out.occ.swap(h.occ);
+    out.hit_rate = h.hit_rate;
     if (target) {
         const StageRec &sr = hs.dev.stages[0];
         out.rot.resize(size_t(sr.n_elem) * 9);

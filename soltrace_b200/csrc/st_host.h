@@ -33,6 +33,8 @@ struct HostScene {
     std::vector<double> inv_cdf;  // table-sunshape inverse CDF (kSunInvCells + 1 entries)
     SceneDev dev;  // stages, sun scalars and flags; device pointers are filled by gpu_run
     uint64_t version = 0;  // another number for every flattened scene of the process, 0: none given
+    // hits per sun ray if no footprint lay over another (at least the true rate), 0 when unknown
+    double hit_rate = 0.0;
     bool has_fe = false;   // an element has a finite-element surface (its queries can fail)
 };
 
@@ -107,6 +109,7 @@ struct SunPosition {
     std::vector<uint32_t> occ;
     std::vector<double> rot;          // tracking: the first stage's re-aimed rotations, 9 per element
                                       // (empty: the scene's elements as they are)
+    double hit_rate = 0.0;            // as HostScene::hit_rate
     uint64_t n_hits = 0;
     uint32_t seed = 0;
 };

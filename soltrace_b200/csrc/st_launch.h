@@ -205,6 +205,7 @@ void launch_list_rank(uint64_t s0, const ProbeOut &o, const uint32_t *offsets, c
 // 215 to 139, beam-down tower 330 to 201; at 130,000 hits the trough would go from 383 to 569
 // (a thread's second ray waits for the longest first one of its warp).
 constexpr uint64_t kSmallRays = 65536;
+constexpr size_t kBatchLanes = 4;  // positions of a batched run in flight at once
 // finite-element interpolation failures flagged by the kernels since the last call
 unsigned take_fe_failures_fp64();
 unsigned take_fe_failures_mixed();

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
+#include <memory>
 #include <thread>
 
 #include "st_host.h"
@@ -77,23 +78,44 @@ cudaError_t upload(DevBuf &b, const std::vector<T> &v, cudaStream_t s, uint64_t 
 
 }  // namespace
 
+// What a batch of sun rays in flight works in: the probe's lists, the sorted hits and the trace's
+// state and queues.
+struct Scratch {
+    DevBuf counts, offsets, total, scan_parts;
+    DevBuf cand;      // probe's ray list: count, then one sun-ray index per entry
+    DevBuf cand_el;   // probe's result per list entry (element + 1, 0 for a miss)
+    DevBuf hit_mask;  // one bit per sun ray of the batch, set for a hit
+    DevBuf amb;       // flat-rectangle probe: count, then the rays left to the double-precision search
+    // trace state and queues (one slot per hit-list entry of a batch)
+    DevBuf wf_sid, wf_raynum, wf_draw, wf_meta, wf_fe0, wf_p, wf_c, wf_t, wf_q0, wf_q1, wf_qs, wf_counts;
+    DevBuf ecount, ecursor, etotal, s_hits;  // the batch's hits sorted by first-stage element (HitRec)
+};
+// One more batch in flight (batched runs), on a stream of its own.
+struct Lane {
+    Scratch scratch;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done = nullptr;
+    ~Lane() {
+        if (done) cudaEventDestroy(done);
+        if (stream) cudaStreamDestroy(stream);
+    }
+    cudaError_t create() {
+        const cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        return e != cudaSuccess ? e : cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    }
+};
+
 // Device buffers, stream and events of one context, kept across runs so that a
 // repeated st_sim_run pays no allocation: every buffer only grows.
-struct Workspace {
+struct Workspace : Scratch {
     int device = -1;
     cudaStream_t stream = nullptr;
     DevBuf stage_cells, grid_sphere, grid_elem, beam_axis, beam_range, beam_elem;
     DevBuf elems, elem_sphere, optics, surf, tables, bvh, bvh_items, cell_start, cell_disc, cell_par, inv_cdf, expos,
         excos;
-    DevBuf acc, ctr, rs, rec_count, counts, offsets, total, scan_parts, recs;
-    DevBuf cand;      // probe's ray list: count, then one sun-ray index per entry
-    DevBuf cand_el;   // probe's result per list entry (element + 1, 0 for a miss)
-    DevBuf hit_mask;  // one bit per sun ray of the batch, set for a hit
-    DevBuf amb;       // mixed probe: count, then the rays left to the double-precision search
-    // trace state and queues (one slot per hit-list entry of a batch)
-    DevBuf wf_sid, wf_raynum, wf_draw, wf_meta, wf_fe0, wf_p, wf_c, wf_t, wf_q0, wf_q1, wf_qs, wf_counts;
+    DevBuf acc, ctr, rs, rec_count, recs;
+    std::vector<std::unique_ptr<Lane>> lanes;  // batched runs: lanes beside this workspace's own scratch
     DevBuf save_rows[2], save_count, replay_rows, replay_fe0;  // stage-data save / replay
-    DevBuf ecount, ecursor, etotal, s_hits;  // the batch's hits sorted by first-stage element (HitRec)
     // record ordering: key counts / slots, scan partials, per-stage counts, merge runs, columns
     DevBuf rec_key, rec_parts, rec_parts2, rec_stage, rec_runs, rec_cols, rec_bad;
     // batched runs: two page-locked staging areas, the positions' tables of a chunk gathered
@@ -159,7 +181,7 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 }  // namespace
 
 // The probe outputs of a batch of n sun rays, in the workspace's buffers.
-static cudaError_t probe_buffers(Workspace &ws, uint64_t n, ProbeOut &o) {
+static cudaError_t probe_buffers(Scratch &ws, uint64_t n, ProbeOut &o) {
     const size_t nb = size_t((n + kProbeBlock - 1) / kProbeBlock);
     cudaError_t e;
     if ((e = ws.counts.ensure(nb * 4)) || (e = ws.cand.ensure((n + 1) * 4)) || (e = ws.cand_el.ensure(n * 4)) ||
@@ -176,9 +198,12 @@ static cudaError_t probe_buffers(Workspace &ws, uint64_t n, ProbeOut &o) {
     return cudaSuccess;
 }
 
+// everything a batch of up to n sun rays on scene S needs
+static cudaError_t batch_buffers(Scratch &ws, const SceneDev &S, uint64_t n);
+
 // trace state and queues for up to `cap` rays: one search queue per search kind among the
 // stages (and round parity)
-static cudaError_t wf_buffers(Workspace &ws, const SceneDev &S, uint64_t cap, WfState &W, WfQueues &Q) {
+static cudaError_t wf_buffers(Scratch &ws, const SceneDev &S, uint64_t cap, WfState &W, WfQueues &Q) {
     cudaError_t e;
     cap = std::max<uint64_t>(cap, 1);
     const int nst = S.n_stages;
@@ -216,6 +241,21 @@ static cudaError_t wf_buffers(Workspace &ws, const SceneDev &S, uint64_t cap, Wf
     W.t = ws.wf_t.as<double>();
     W.cap = uint32_t(cap);
     return cudaSuccess;
+}
+
+static cudaError_t batch_buffers(Scratch &ws, const SceneDev &S, uint64_t n) {
+    const uint32_t nb = uint32_t((n + kProbeBlock - 1) / kProbeBlock);
+    const size_t n_elem = size_t(std::max(S.stages[0].n_elem, 1)) * 4;
+    ProbeOut po;
+    WfState W;
+    WfQueues Q;
+    cudaError_t e;
+    if ((e = probe_buffers(ws, n, po)) || (e = ws.offsets.ensure(size_t(nb) * 4)) ||
+        (e = ws.scan_parts.ensure(scan_parts(nb) * 4)) || (e = ws.total.ensure(8)) ||
+        (e = ws.s_hits.ensure(n * sizeof(HitRec))) || (e = ws.ecount.ensure(n_elem)) ||
+        (e = ws.ecursor.ensure(n_elem)) || (e = ws.etotal.ensure(8)))
+        return e;
+    return wf_buffers(ws, S, n, W, Q);
 }
 
 // TRayData::Merge (types.cpp:311-355): a stage's records are kept in blocks of 8192; merging
@@ -651,7 +691,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         };
         uint64_t sun_next = 0;
         uint64_t global_done = 0;  // over several ranks: hits numbered by all ranks so far
-        double p_est = rq.hit_rate_hint > 0 ? rq.hit_rate_hint : 0.0;
+        // hits per sun ray: the last run's, or the scene's estimate, or (0) a pilot batch's
+        double p_est = rq.hit_rate_hint > 0 ? rq.hit_rate_hint : multi ? 0.0 : hs.hit_rate / 1.05;
         RunState rs = rs0;
         size_t ev_used = 0;
         auto new_event = [&]() {
@@ -1381,26 +1422,20 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     CK(ws.rec_count.ensure(8));
     for (auto &O : Op) O.rec_count = ws.rec_count.as<unsigned long long>();
 
-    // buffers for the largest batch, sized before anything is queued (growing a buffer frees
-    // the old one, which must not happen under queued work)
-    const uint64_t kMaxBatch = uint64_t(1) << 26;
+    // Positions run on kBatchLanes lanes (streams with scratch of their own) in turn: a position's
+    // kernels number a few hundred thousand rays and leave most of the GPU idle at their ends,
+    // which another position's kernels fill.  Four lanes of batches of at most 2^24 sun rays take
+    // the memory of one lane of 2^26.  Lane 0 is the workspace's own scratch and stream.  24 sun
+    // positions of a 2,000-heliostat beam-down field (250,000 hits each): 21.7 ms of device time
+    // on one lane in two waves, 7.2 on four in one.
     const uint32_t n_elem0 = uint32_t(S0.stages[0].n_elem);
-    {
-        const uint64_t n = kMaxBatch;
-        const uint32_t nb = uint32_t((n + kProbeBlock - 1) / kProbeBlock);
-        ProbeOut po;
-        WfState W;
-        WfQueues Q;
-        CK(probe_buffers(ws, n, po));
-        CK(ws.offsets.ensure(size_t(nb) * 4));
-        CK(ws.scan_parts.ensure(scan_parts(nb) * 4));
-        CK(ws.total.ensure(8));
-        CK(ws.s_hits.ensure(n * sizeof(HitRec)));
-        CK(ws.ecount.ensure(size_t(std::max<uint32_t>(n_elem0, 1)) * 4));
-        CK(ws.ecursor.ensure(size_t(std::max<uint32_t>(n_elem0, 1)) * 4));
-        CK(ws.etotal.ensure(8));
-        CK(wf_buffers(ws, S0, n, W, Q));
+    const size_t n_lanes = std::min<size_t>(K, kBatchLanes);
+    const uint64_t kMaxBatch = uint64_t(1) << (n_lanes > 1 ? 24 : 26);
+    while (ws.lanes.size() + 1 < n_lanes) {
+        ws.lanes.push_back(std::make_unique<Lane>());
+        CK(ws.lanes.back()->create());
     }
+    for (auto &l : ws.lanes) CK(cudaStreamSynchronize(l->stream));  // idle, unless a run failed
     CK(cudaStreamSynchronize(st));
     out.setup_ms = ms_since(t_setup);
 
@@ -1419,6 +1454,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     RunState *drs = ws.pos_rs.as<RunState>();
     std::vector<uint64_t> sun_next(K, 0);
     std::vector<double> p_est(K, 0.0);
+    for (size_t p = 0; p < K; ++p) p_est[p] = pos[p].hit_rate / 1.05;  // an upper estimate (0: none)
     std::vector<bool> reached(K, false);
     size_t left = K;
     for (size_t p = 0; p < K; ++p)
@@ -1426,8 +1462,10 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
             reached[p] = true;
             --left;
         }
+    std::vector<uint64_t> wants(K, 0);
     while (left > 0) {
         out.waves++;
+        uint64_t largest = 0;
         for (size_t p = 0; p < K; ++p) {
             if (reached[p]) continue;
             uint64_t want;
@@ -1443,6 +1481,18 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 out.error = buf;
                 return false;
             }
+            wants[p] = want;
+            largest = std::max(largest, std::min(want, kMaxBatch));
+        }
+        // room for the wave's largest batch in every lane, before anything is queued (growing a
+        // buffer frees the old one, which must not happen under queued work)
+        for (size_t l = 0; l < n_lanes; ++l)
+            CK(batch_buffers(l ? ws.lanes[l - 1]->scratch : static_cast<Scratch &>(ws), S0, largest));
+        for (size_t p = 0; p < K; ++p) {
+            if (reached[p]) continue;
+            const uint64_t want = wants[p], need = pos[p].n_hits - rs_h[p].hits_done;
+            Scratch &sc = p % n_lanes ? ws.lanes[p % n_lanes - 1]->scratch : static_cast<Scratch &>(ws);
+            cudaStream_t st = p % n_lanes ? ws.lanes[p % n_lanes - 1]->stream : ws.stream;
             const SceneDev &S = Sp[p];
             for (uint64_t queued = 0; queued < want;) {
                 const uint64_t n = std::min<uint64_t>(kMaxBatch, want - queued);
@@ -1450,8 +1500,8 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 ProbeOut po;
                 WfState W;
                 WfQueues Q;
-                CK(probe_buffers(ws, n, po));
-                CK(wf_buffers(ws, S, n, W, Q));
+                CK(probe_buffers(sc, n, po));
+                CK(wf_buffers(sc, S, n, W, Q));
                 cudaEvent_t p0 = new_event(), p1 = new_event(), p2 = new_event();
                 CK(cudaEventRecord(p0, st));
                 const uint64_t s0 = sun_next[p];
@@ -1459,29 +1509,29 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                     out.gpu_launches += launch_probe_mixed(S, s0, uint32_t(n), po, drs + p, st);
                 else
                     out.gpu_launches += launch_probe_fp64(S, s0, uint32_t(n), po, drs + p, st);
-                out.gpu_launches += launch_scan(po.block_counts, nb, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(),
-                                                ws.scan_parts.as<uint32_t>(), st);
+                out.gpu_launches += launch_scan(po.block_counts, nb, sc.offsets.as<uint32_t>(), sc.total.as<uint32_t>(),
+                                                sc.scan_parts.as<uint32_t>(), st);
                 if (std::min<uint64_t>(n, need) <= kSmallRays) {
-                    launch_list_rank(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p,
-                                     ws.s_hits.as<HitRec>(), uint32_t(n), st);
+                    launch_list_rank(s0, po, sc.offsets.as<uint32_t>(), sc.total.as<uint32_t>(), drs + p,
+                                     sc.s_hits.as<HitRec>(), uint32_t(n), st);
                     out.gpu_launches += 1;
                     Q.rounds = 0;
                 } else {
-                    launch_list_sort(s0, po, ws.offsets.as<uint32_t>(), ws.total.as<uint32_t>(), drs + p, n_elem0,
-                                     ws.ecount.as<uint32_t>(), ws.ecursor.as<uint32_t>(), ws.etotal.as<uint32_t>(),
-                                     ws.s_hits.as<HitRec>(),
+                    launch_list_sort(s0, po, sc.offsets.as<uint32_t>(), sc.total.as<uint32_t>(), drs + p, n_elem0,
+                                     sc.ecount.as<uint32_t>(), sc.ecursor.as<uint32_t>(), sc.etotal.as<uint32_t>(),
+                                     sc.s_hits.as<HitRec>(),
                                      uint32_t(n), st);
                     out.gpu_launches += 3;
                 }
                 CK(cudaEventRecord(p1, st));
                 if (rq.precision)
-                    out.gpu_launches += launch_trace_mixed(false, S, ws.s_hits.as<HitRec>(), ws.total.as<uint32_t>(), drs + p,
+                    out.gpu_launches += launch_trace_mixed(false, S, sc.s_hits.as<HitRec>(), sc.total.as<uint32_t>(), drs + p,
                                                            Op[p], W, Q, nullptr, st);
                 else
-                    out.gpu_launches += launch_trace_fp64(false, S, ws.s_hits.as<HitRec>(), ws.total.as<uint32_t>(), drs + p,
+                    out.gpu_launches += launch_trace_fp64(false, S, sc.s_hits.as<HitRec>(), sc.total.as<uint32_t>(), drs + p,
                                                           Op[p], W, Q, nullptr, st);
                 CK(cudaEventRecord(p2, st));
-                launch_advance(ws.total.as<uint32_t>(), nullptr, s0, uint32_t(n), drs + p, st);
+                launch_advance(sc.total.as<uint32_t>(), nullptr, s0, uint32_t(n), drs + p, st);
                 CK(cudaGetLastError());
                 out.gpu_launches += 1;
                 probe_ev.push_back({p0, p1});
@@ -1490,6 +1540,10 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
                 sun_next[p] += n;
                 out.batches++;
             }
+        }
+        for (size_t l = 1; l < n_lanes; ++l) {  // the read-back below waits for every lane
+            CK(cudaEventRecord(ws.lanes[l - 1]->done, ws.lanes[l - 1]->stream));
+            CK(cudaStreamWaitEvent(st, ws.lanes[l - 1]->done, 0));
         }
         CK(cudaMemcpyAsync(rs_h.data(), drs, K * sizeof(RunState), cudaMemcpyDeviceToHost, st));
         out.d2h_bytes += K * sizeof(RunState);
@@ -1518,6 +1572,12 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         float x = 0;
         cudaEventElapsedTime(&x, pe.first, pe.second);
         out.trace_ms += x;
+    }
+    // the lanes' times overlap: scaled, so that they stay a split of the device time
+    const double both = out.probe_ms + out.trace_ms;
+    if (n_lanes > 1 && both > out.device_ms) {
+        out.probe_ms *= out.device_ms / both;
+        out.trace_ms *= out.device_ms / both;
     }
     std::vector<RunCounters> ctr(K);
     std::vector<unsigned long long> accv(K * acc_n);
