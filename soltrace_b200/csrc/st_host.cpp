@@ -1009,7 +1009,6 @@ struct OccupancyMap {
             stride = (nx + 31) / 32;
             if (size_t(stride) * size_t(ny) <= size_t(kMaxOccWords) || k <= -9) break;
         }
-        bits.assign(size_t(stride) * size_t(ny), 0u);
         side = ldexp(cell, -k);
         pad = 4.0 * fp.eps;
     }
@@ -1036,20 +1035,47 @@ struct OccupancyMap {
 };
 
 // ---------------- the sun frame and sun box (suntoprimarystage.cpp:59-293) ----------------
-bool sun_setup(Context *cx, HostScene &hs) {
-    StageM &st = cx->stages[0];
-    SunM &sun = cx->sun;
+// the fields of SunDev that place the sun-plane grid, and those of the flat-rectangle probe
+void grid_fields(SunDev &sd, const SunM &sun, double cell, int nx, int ny) {
+    sd.grid_on = 1;
+    sd.gnx = nx;
+    sd.gny = ny;
+    sd.gx0 = sun.xmin;
+    sd.gy0 = sun.ymin;
+    sd.ginv = 1.0 / cell;
+    sd.gcell = cell;
+}
+void flat_probe_fields(SunDev &sd, const FlatProbe &fp, const OccupancyMap &occ, double cell) {
+    sd.fx_mul = fp.mul[0];
+    sd.fy_mul = fp.mul[1];
+    sd.fx_shift = fp.shift[0];
+    sd.fy_shift = fp.shift[1];
+    sd.fcell = float(cell);
+    sd.occ_shx = fp.shift[0] - occ.k;
+    sd.occ_shy = fp.shift[1] - occ.k;
+    sd.occ_stride = occ.stride;
+    sd.occ_words = occ.stride * occ.ny;
+}
+// cell size of the sun-plane grid over a W x H box (elements of radius rmax at most) within a
+// budget of cells
+double sun_cell_size(double W, double H, double rmax, double budget) {
+    double cell = std::max(rmax * 0.5, 1e-6);
+    while ((W / cell + 1) * (H / cell + 1) > budget) cell *= 1.5;
+    return cell;
+}
+
+// Sun frame and sun box over the enabled elements of the first stage, and the sun's scalars
+// (suntoprimarystage.cpp:59-293); Rs the stage -> sun rotation.  Empty, or the error's message.
+std::string sun_frame(const StageM &st, SunM &sun, SunDev &sd, double Rs[9]) {
     const double dx = 0.0 - sun.origin[0], dy = 0.0 - sun.origin[1], dz = 0.0 - sun.origin[2];
     const double dt = sqrt(dx * dx + dy * dy + dz * dz);
     if (dt == 0.0) {
-        cx->log("error calculating sun position in primary stage, dtot = 0.0\n");
-        return false;
+        return "error calculating sun position in primary stage, dtot = 0.0\n";
     }
     const double cg[3] = {dx / dt, dy / dt, dz / dt};
     double cs[3];
     mulv(st.R, cg, cs);
     const double se[3] = {atan2(cs[0], cs[2]), asin(cs[1]), 0.0};
-    double Rs[9];
     rot_from_euler(se, Rs);
     sun.xmax = -1.0e20;
     sun.xmin = 1.0e20;
@@ -1110,10 +1136,8 @@ bool sun_setup(Context *cx, HostScene &hs) {
         n++;
     }
     if (n == 0) {
-        cx->log("error calculating sun position in primary stage because no elements were enabled");
-        return false;
+        return "error calculating sun position in primary stage because no elements were enabled";
     }
-    SunDev &sd = hs.dev.sun;
     sd.xmin = sun.xmin;
     sd.xmax = sun.xmax;
     sd.ymin = sun.ymin;
@@ -1126,6 +1150,19 @@ bool sun_setup(Context *cx, HostScene &hs) {
     sd.shape = sun.shape;
     sd.point_source = sun.point_source ? 1 : 0;
     sd.sigma = sun.sigma;
+    return "";
+}
+
+bool sun_setup(Context *cx, HostScene &hs) {
+    StageM &st = cx->stages[0];
+    SunM &sun = cx->sun;
+    SunDev &sd = hs.dev.sun;
+    double Rs[9];
+    const std::string err = sun_frame(st, sun, sd, Rs);
+    if (!err.empty()) {
+        cx->log("%s", err.c_str());
+        return false;
+    }
 
     // Inverse CDF of p(theta) ~ theta * I(theta) on [0, MaxAngle] for table sunshapes:
     // trapezoid CDF on kSunCdfCells cells, then theta(u) tabulated at kSunInvCells + 1
@@ -1197,9 +1234,8 @@ bool sun_setup(Context *cx, HostScene &hs) {
         }
         if (bounded && rmax > 0) {
             const double W = sun.xmax - sun.xmin, H = sun.ymax - sun.ymin;
-            double cell = std::max(rmax * 0.5, 1e-6);
-            // keep the grid within the context's cell budget (~4M cells for a single run)
-            while ((W / cell + 1) * (H / cell + 1) > cx->sun_grid_cells) cell *= 1.5;
+            // within the context's cell budget (~4M cells for a single run)
+            const double cell = sun_cell_size(W, H, rmax, cx->sun_grid_cells);
             const int nx = std::max(1, int(ceil(W / cell))), ny = std::max(1, int(ceil(H / cell)));
             const FlatProbe fp = flat_probe_params(W, H, cell, rmax, st.elems, Rs);
             // Per element a float disc (centre, radius) and a parallelogram about the same
@@ -1263,11 +1299,14 @@ bool sun_setup(Context *cx, HostScene &hs) {
             }
             // Cells: an element is listed where both its disc and its parallelogram reach (the second
             // leaves a third of the disc's cells on a heliostat field); elements that accept no hit
-            // (disabled, or flat beyond their ZAperture, element_test_flat) are listed nowhere.
+            // (disabled; flat beyond their ZAperture or of negative size, element_test_flat) are listed
+            // nowhere.
             bool exact = fp.ok;
             for (const Elem &e : st.elems)
                 if (e.stype != 3 || char(tolower(e.shape)) != 'r') exact = false;
-            auto never = [&](const Elem &e) { return !e.enabled || (exact && !(0.0 <= e.zap)); };
+            auto never = [&](const Elem &e) {
+                return !e.enabled || (exact && (!(0.0 <= e.zap) || e.p[0] < 0.0 || e.p[1] < 0.0));
+            };
             std::vector<std::vector<int>> cells(size_t(nx) * ny);
             for (size_t j = 0; j < st.elems.size(); ++j) {
                 if (never(st.elems[j])) continue;
@@ -1301,7 +1340,10 @@ bool sun_setup(Context *cx, HostScene &hs) {
             // projected along the sun's z, inverted).  Coordinates are taken relative to the
             // lower corner of the entry's cell, so that floats hold them to ~1e-6 m.
             OccupancyMap occ;
-            if (exact) occ.size(nx, ny, cell, fp);
+            if (exact) {
+                occ.size(nx, ny, cell, fp);
+                occ.bits.assign(size_t(occ.stride) * size_t(occ.ny), 0u);
+            }
             std::vector<float4> xb(exact ? st.elems.size() : 0), xc(exact ? st.elems.size() : 0);
             std::vector<float> xtol(exact ? st.elems.size() : 0, 0.f);
             std::vector<double> ecx(exact ? st.elems.size() : 0), ecy(exact ? st.elems.size() : 0);
@@ -1365,24 +1407,10 @@ bool sun_setup(Context *cx, HostScene &hs) {
             }
             sd.exact_flat = exact ? 1 : 0;
             if (exact) {
-                sd.fx_mul = fp.mul[0];
-                sd.fy_mul = fp.mul[1];
-                sd.fx_shift = fp.shift[0];
-                sd.fy_shift = fp.shift[1];
-                sd.fcell = float(cell);
-                sd.occ_shx = fp.shift[0] - occ.k;
-                sd.occ_shy = fp.shift[1] - occ.k;
-                sd.occ_stride = occ.stride;
-                sd.occ_words = int(occ.bits.size());
+                flat_probe_fields(sd, fp, occ, cell);
                 hs.occ.swap(occ.bits);
             }
-            sd.grid_on = 1;
-            sd.gnx = nx;
-            sd.gny = ny;
-            sd.gx0 = sun.xmin;
-            sd.gy0 = sun.ymin;
-            sd.ginv = 1.0 / cell;
-            sd.gcell = cell;
+            grid_fields(sd, sun, cell, nx, ny);
         }
     }
     return true;
@@ -1812,12 +1840,116 @@ int run(Context *cx, unsigned seed) {
 constexpr double kBatchSunGridCells = 2.5e5;
 constexpr size_t kBatchChunk = 64;
 
+// A tracking element's aim point and rotation for one sun position
+struct Tracker {
+    double s[3], target[3];
+    std::string set(const double sun_xyz[3], const double tgt[3]) {
+        const double sn = sqrt(sq(sun_xyz[0]) + sq(sun_xyz[1]) + sq(sun_xyz[2]));
+        if (!(sn > 0)) return "sun position at the origin";
+        for (int q = 0; q < 3; ++q) {
+            s[q] = sun_xyz[q] / sn;
+            target[q] = tgt[q];
+        }
+        return "";
+    }
+    std::string aim(const Elem &e, double aim_pt[3], double R[9]) const {
+        double t[3] = {target[0] - e.origin[0], target[1] - e.origin[1], target[2] - e.origin[2]};
+        const double tn = sqrt(sq(t[0]) + sq(t[1]) + sq(t[2]));
+        double n[3];
+        for (int q = 0; q < 3; ++q) n[q] = s[q] + (tn > 0 ? t[q] / tn : 0.0);
+        const double nn = sqrt(sq(n[0]) + sq(n[1]) + sq(n[2]));
+        if (!(nn > 0)) return "a tracking element cannot bisect the sun and target directions";
+        for (int q = 0; q < 3; ++q) aim_pt[q] = e.origin[q] + 100.0 * (n[q] / nn);
+        double eu[3];
+        if (!euler_of(e.origin, aim_pt, e.zrot, eu)) return "a tracking element's geometry is not possible";
+        rot_from_euler(eu, R);
+        return "";
+    }
+};
+
+// Whether a batched run's sun-plane grids can be built on the device: flat rectangles of bounded
+// size under a distant sun.
+bool device_grids_ok(const Context *cx) {
+    const StageM &st = cx->stages[0];
+    if (cx->sun.point_source || st.elems.size() < 4) return false;
+    double rmax = 0.0;
+    for (const Elem &e : st.elems) {
+        if (e.stype != 3 || char(tolower(e.shape)) != 'r') return false;
+        const double r = accept_radius(e);
+        if (r < 0) return false;
+        rmax = std::max(rmax, r);
+    }
+    return rmax > 0;
+}
+
+// The part of a position that the host makes when the device builds its grid: sun frame and box,
+// rotations, and the grid's geometry.  out.on_device stays false when this position's box has no
+// fixed-point scale (FlatProbe::ok).
+bool build_position_frame(const Context *cx, const HostScene &hs, const double sun_xyz[3], const double *target,
+                          SunPosition &out, std::string &err) {
+    const StageM &st = cx->stages[0];
+    SunM sun = cx->sun;
+    for (int q = 0; q < 3; ++q) sun.origin[q] = sun_xyz[q];
+    out.sun = hs.dev.sun;
+    double Rs[9];
+    if (!(err = sun_frame(st, sun, out.sun, Rs)).empty()) return false;
+    double rmax = 0.0;
+    for (const Elem &e : st.elems) rmax = std::max(rmax, accept_radius(e));
+    const double W = sun.xmax - sun.xmin, H = sun.ymax - sun.ymin;
+    const double cell = sun_cell_size(W, H, rmax, kBatchSunGridCells);
+    const int nx = std::max(1, int(ceil(W / cell))), ny = std::max(1, int(ceil(H / cell)));
+    const FlatProbe fp = flat_probe_params(W, H, cell, rmax, st.elems, Rs);
+    if (!fp.ok) return true;
+    OccupancyMap occ;
+    occ.size(nx, ny, cell, fp);
+    grid_fields(out.sun, sun, cell, nx, ny);
+    flat_probe_fields(out.sun, fp, occ, cell);
+    out.sun.exact_flat = 1;
+    PosGrid &g = out.grid;
+    for (int q = 0; q < 9; ++q) g.Rs[q] = Rs[q];
+    g.x0 = sun.xmin;
+    g.y0 = sun.ymin;
+    g.cell = cell;
+    g.eps = fp.eps;
+    g.box_ext = fabs(sun.xmin) + fabs(sun.xmax) + fabs(sun.ymin) + fabs(sun.ymax);
+    g.side = occ.side;
+    g.pad = occ.pad;
+    g.nx = nx;
+    g.ny = ny;
+    g.onx = occ.nx;
+    g.ony = occ.ny;
+    g.ostride = occ.stride;
+    Tracker tr;
+    if (target) {
+        if (!(err = tr.set(sun_xyz, target)).empty()) return false;
+        out.rot.resize(st.elems.size() * 9);
+    }
+    for (size_t k = 0; k < st.elems.size(); ++k) {
+        const Elem &e = st.elems[k];
+        const double *R = e.R;
+        if (target) {
+            double aim_pt[3];
+            if (!(err = tr.aim(e, aim_pt, &out.rot[9 * k])).empty()) return false;
+            R = &out.rot[9 * k];
+        }
+        if (!e.enabled || !(0.0 <= e.zap) || e.p[0] < 0.0 || e.p[1] < 0.0) continue;
+        // |det| of the projected half-axes is their product times the sun's cosine on the plane
+        double nz[3];
+        mulv(Rs, R + 6, nz);
+        out.hit_rate += fabs(e.p[0] * e.p[1] * nz[2]) / (W * H);
+    }
+    out.hit_rate = std::min(out.hit_rate, 1.0);
+    out.on_device = true;
+    return true;
+}
+
 // The sun-dependent tables of one position of a batched run: the context's sun moved to
 // `sun_xyz` and, with `target`, every first-stage element re-aimed so that its normal bisects
 // the sun direction and the direction to the target (a heliostat tracking the sun; the aim
 // point is origin + 100 n, zrot kept, rotation by input.cpp:160-176).
 bool build_position(const Context *cx, const HostScene &hs, const double sun_xyz[3], const double *target,
-                    SunPosition &out, std::string &err) {
+                    bool device_grids, SunPosition &out, std::string &err) {
+    if (device_grids) return build_position_frame(cx, hs, sun_xyz, target, out, err);
     Context c;
     c.sun = cx->sun;
     c.sun_grid_cells = kBatchSunGridCells;
@@ -1827,30 +1959,10 @@ bool build_position(const Context *cx, const HostScene &hs, const double sun_xyz
     c.stages.push_back(cx->stages[0]);
     StageM &st0 = c.stages[0];
     if (target) {
-        const double sn = sqrt(sq(sun_xyz[0]) + sq(sun_xyz[1]) + sq(sun_xyz[2]));
-        if (!(sn > 0)) {
-            err = "sun position at the origin";
-            return false;
-        }
-        const double s[3] = {sun_xyz[0] / sn, sun_xyz[1] / sn, sun_xyz[2] / sn};
-        for (Elem &e : st0.elems) {
-            double t[3] = {target[0] - e.origin[0], target[1] - e.origin[1], target[2] - e.origin[2]};
-            const double tn = sqrt(sq(t[0]) + sq(t[1]) + sq(t[2]));
-            double n[3];
-            for (int q = 0; q < 3; ++q) n[q] = s[q] + (tn > 0 ? t[q] / tn : 0.0);
-            const double nn = sqrt(sq(n[0]) + sq(n[1]) + sq(n[2]));
-            if (!(nn > 0)) {
-                err = "a tracking element cannot bisect the sun and target directions";
-                return false;
-            }
-            for (int q = 0; q < 3; ++q) e.aim[q] = e.origin[q] + 100.0 * (n[q] / nn);
-            double eu[3];
-            if (!euler_of(e.origin, e.aim, e.zrot, eu)) {
-                err = "a tracking element's geometry is not possible";
-                return false;
-            }
-            rot_from_euler(eu, e.R);
-        }
+        Tracker tr;
+        if (!(err = tr.set(sun_xyz, target)).empty()) return false;
+        for (Elem &e : st0.elems)
+            if (!(err = tr.aim(e, e.aim, e.R)).empty()) return false;
     }
     HostScene h;
     h.dev = hs.dev;
@@ -1904,8 +2016,8 @@ int run_batch(Context *cx, unsigned seed, int n_pos, const double *sun_xyz, cons
     for (auto &f : cx->flux) rq.flux.push_back(f.req);
     // positions go to the device in chunks; the host builds the next chunk's tables while
     // the device runs the current one
-    auto build_chunk = [cx, &hs, sun_xyz, hits, target, seed](size_t a, size_t b, std::vector<SunPosition> &pos,
-                                                               std::string &err) -> bool {
+    auto build_all = [cx, &hs, sun_xyz, hits, target, seed](size_t a, size_t b, bool device_grids,
+                                                            std::vector<SunPosition> &pos, std::string &err) -> bool {
         const size_t n = b - a;
         pos.assign(n, SunPosition());
         std::vector<std::string> errs(n);
@@ -1916,7 +2028,7 @@ int run_batch(Context *cx, unsigned seed, int n_pos, const double *sun_xyz, cons
             th.emplace_back([&, t]() {
                 for (size_t i = t; i < n; i += nth) {
                     const size_t p = a + i;
-                    ok[i] = build_position(cx, hs, sun_xyz + 3 * p, target, pos[i], errs[i]);
+                    ok[i] = build_position(cx, hs, sun_xyz + 3 * p, target, device_grids, pos[i], errs[i]);
                     pos[i].n_hits = uint64_t(hits[p]);
                     pos[i].seed = seed + unsigned(p);
                 }
@@ -1927,6 +2039,14 @@ int run_batch(Context *cx, unsigned seed, int n_pos, const double *sun_xyz, cons
                 err = "sun position " + std::to_string(a + i) + ": " + errs[i];
                 return false;
             }
+        return true;
+    };
+    // a chunk's grids are all built on the device, or all here
+    const bool flat = device_grids_ok(cx);
+    auto build_chunk = [&build_all, flat](size_t a, size_t b, std::vector<SunPosition> &pos, std::string &err) -> bool {
+        if (!build_all(a, b, flat, pos, err)) return false;
+        for (const SunPosition &p : pos)
+            if (flat && !p.on_device) return build_all(a, b, false, pos, err);
         return true;
     };
     if (!cx->ws) cx->ws = workspace_create();

@@ -7,6 +7,7 @@
 
 #include <vector_types.h>
 
+#include "st_launch.h"
 #include "st_scene.h"
 
 namespace stb {
@@ -110,6 +111,8 @@ struct SunPosition {
     std::vector<double> rot;          // tracking: the first stage's re-aimed rotations, 9 per element
                                       // (empty: the scene's elements as they are)
     double hit_rate = 0.0;            // as HostScene::hit_rate
+    bool on_device = false;           // grid, footprints and bitmap are built on the device from
+    PosGrid grid{};                   // this (element table and offsets filled by gpu_run_batch)
     uint64_t n_hits = 0;
     uint32_t seed = 0;
 };

@@ -251,6 +251,42 @@ void launch_rec_scatter(const RecOrder &o, cudaStream_t st);
 // rotation rot[9e .. 9e + 8]
 void launch_set_rotations(ElemRec *el, uint32_t n, const double *rot, cudaStream_t st);
 
+// Sun-plane grids of a batched run's positions, built on the device (first stages of flat
+// rectangles): what sun_setup builds on the host for a single run, from the element records the
+// position traces with.  Positions' cells, bitmaps and entries lie end to end; cell ranges index
+// the entries of all positions.
+struct PosGrid {
+    double Rs[9];                 // sun frame
+    double x0, y0, cell;          // lower corner of the sun box, cell size
+    double eps, box_ext;          // FlatProbe::eps; |xmin| + |xmax| + |ymin| + |ymax|
+    double side, pad;             // occupancy bitmap: side of its squares, widening
+    const ElemRec *elems;         // the position's element table (first stage at first_elem)
+    int nx, ny;                   // cells
+    int onx, ony, ostride;        // bitmap squares, words a row
+    uint32_t cell0, occ0;         // first cell, first bitmap word
+};
+// One element's footprint in one position's sun plane, float fields as SunDev's entries hold them
+struct PosFoot {
+    double cx, cy, pad;           // centre, radius of the listing test
+    float4 disc, par, xb, xc;
+    float xtol;
+    int x0, x1, y0, y1;           // cells the disc may reach (x1 < x0: listed nowhere)
+};
+struct PosGridBuild {
+    const PosGrid *grids;
+    int n_pos, n_elem, first_elem;
+    uint32_t n_cells;             // of all positions
+    PosFoot *feet;                // n_pos * n_elem
+    uint32_t *counts, *offsets, *cursor;  // per cell
+    uint32_t *list;               // entries: element, then (sorted per cell) written out below
+    uint32_t n_entries;           // room in list and the arrays below
+    int2 *cells;
+    float4 *disc, *par, *xa, *xb, *xc;
+    uint32_t *occ;
+};
+void launch_pos_footprints(const PosGridBuild &b, cudaStream_t st);  // feet, counts, occ
+void launch_pos_entries(const PosGridBuild &b, cudaStream_t st);     // list, cells, entry arrays
+
 void launch_compact(uint64_t s0, uint32_t n, const uint32_t *hit_elem, const uint32_t *counts,
                     const uint32_t *offsets, uint64_t *hit_sid, uint32_t *hit_el, cudaStream_t st);
 // cut-off and run state after a batch; the last numbered sun ray is read from the

@@ -128,7 +128,8 @@ struct Workspace : Scratch {
     size_t rec_host_bytes = 0;
     bool rec_host_pinned = false;
     // batched runs: per-position sun tables, element copies, run states, counters, accumulators
-    DevBuf pos_cells, pos_disc, pos_par, pos_xa, pos_xb, pos_xc, pos_occ, pos_elems, pos_rot, pos_rs, pos_ctr, pos_acc;
+    DevBuf pos_cells, pos_disc, pos_par, pos_xa, pos_xb, pos_xc, pos_occ, pos_elems, pos_grids, pos_feet, pos_counts, pos_offsets, pos_cursor, pos_list, pos_parts, pos_parts2,
+        pos_total, pos_rot, pos_rs, pos_ctr, pos_acc;
     DevBuf cell_xa, cell_xb, cell_xc, occ;  // exact flat footprints of the sun-plane grid
     std::vector<cudaEvent_t> events;
     // the scene whose tables the buffers above hold (HostScene::version), 0 for none: a run on
@@ -1246,7 +1247,8 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     // every position's tables, laid end to end on the device: sized first, then each position's
     // arrays copied straight from its own vectors (no host-side concatenation)
     std::vector<size_t> off_cells(K), off_disc(K), off_elems(K), off_rot(K);
-    bool all_exact = true;
+    bool all_exact = true, on_device = true;  // (a chunk's positions are built alike)
+    for (const SunPosition &sp : pos) on_device = on_device && sp.on_device;
     for (const SunPosition &sp : pos)
         if (!sp.sun.exact_flat || sp.cell_xa.size() != sp.cell_disc.size() || sp.cell_xa.empty()) all_exact = false;
     const size_t n_elem_all = hs.elems.size(), n_first = size_t(hs.dev.stages[0].n_elem);
@@ -1329,6 +1331,70 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         }
     }
 
+    std::vector<PosGrid> grids;
+    if (on_device) {
+        // every position's grid: footprints and counts, their scan, then the entries
+        uint64_t cells = 0, words = 0;
+        for (size_t p = 0; p < K; ++p) {
+            PosGrid g = pos[p].grid;
+            g.elems = (off_elems[p] != size_t(-1) ? ws.pos_elems.as<ElemRec>() + off_elems[p] : ws.elems.as<ElemRec>());
+            g.cell0 = uint32_t(cells);
+            g.occ0 = uint32_t(words);
+            cells += uint64_t(g.nx) * uint64_t(g.ny);
+            words += uint64_t(pos[p].sun.occ_words);
+            grids.push_back(g);
+        }
+        const uint32_t nc = uint32_t(cells);
+        CK(ws.pos_grids.ensure(K * sizeof(PosGrid)));
+        CK(ws.pos_feet.ensure(K * n_first * sizeof(PosFoot)));
+        CK(ws.pos_counts.ensure(cells * 4));
+        CK(ws.pos_offsets.ensure(cells * 4));
+        CK(ws.pos_cursor.ensure(cells * 4));
+        CK(ws.pos_cells.ensure(cells * sizeof(int2)));
+        CK(ws.pos_occ.ensure(words * 4));
+        CK(ws.pos_parts.ensure(scan_parts(nc) * 4));
+        CK(ws.pos_parts2.ensure(scan_parts(uint32_t(scan_parts(nc))) * 4));
+        CK(ws.pos_total.ensure(8));
+        CK(put(ws.pos_grids, 0, grids.data(), K * sizeof(PosGrid)));
+        CK(cudaMemsetAsync(ws.pos_counts.p, 0, cells * 4, st));
+        CK(cudaMemsetAsync(ws.pos_cursor.p, 0, cells * 4, st));
+        CK(cudaMemsetAsync(ws.pos_occ.p, 0, words * 4, st));
+        PosGridBuild b{};
+        b.grids = ws.pos_grids.as<PosGrid>();
+        b.n_pos = int(K);
+        b.n_elem = int(n_first);
+        b.first_elem = hs.dev.stages[0].first_elem;
+        b.n_cells = nc;
+        b.feet = ws.pos_feet.as<PosFoot>();
+        b.counts = ws.pos_counts.as<uint32_t>();
+        b.offsets = ws.pos_offsets.as<uint32_t>();
+        b.cursor = ws.pos_cursor.as<uint32_t>();
+        b.occ = ws.pos_occ.as<uint32_t>();
+        launch_pos_footprints(b, st);
+        launch_scan_large(b.counts, nc, b.offsets, ws.pos_total.as<uint32_t>(), ws.pos_parts.as<uint32_t>(),
+                          ws.pos_parts2.as<uint32_t>(), st);
+        uint32_t total = 0;
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&total, ws.pos_total.p, 4, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        b.n_entries = total;
+        CK(ws.pos_list.ensure(std::max<size_t>(size_t(total) * 4, 16)));
+        for (DevBuf *d : {&ws.pos_disc, &ws.pos_par, &ws.pos_xa, &ws.pos_xb, &ws.pos_xc})
+            CK(d->ensure(std::max<size_t>(size_t(total) * sizeof(float4), 16)));
+        b.list = ws.pos_list.as<uint32_t>();
+        b.cells = ws.pos_cells.as<int2>();
+        b.disc = ws.pos_disc.as<float4>();
+        b.par = ws.pos_par.as<float4>();
+        b.xa = ws.pos_xa.as<float4>();
+        b.xb = ws.pos_xb.as<float4>();
+        b.xc = ws.pos_xc.as<float4>();
+        CK(cudaMemsetAsync(ws.pos_list.p, 0, size_t(total) * 4, st));
+        launch_pos_entries(b, st);
+        CK(cudaGetLastError());
+        out.gpu_launches += 8;
+        all_exact = true;
+    }
+
     SceneDev S0 = hs.dev;
     S0.elems = ws.elems.as<ElemRec>();
     S0.elem_sphere = ws.elem_sphere.as<float4>();
@@ -1380,14 +1446,14 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     for (size_t p = 0; p < K; ++p) {
         SceneDev &S = Sp[p];
         S.sun = pos[p].sun;
-        S.sun.cell_start = ws.pos_cells.as<int>() + off_cells[p];
+        S.sun.cell_start = ws.pos_cells.as<int>() + (on_device ? 2 * size_t(grids[p].cell0) : off_cells[p]);
         S.sun.cell_disc = ws.pos_disc.as<float4>() + off_disc[p];
         S.sun.cell_par = ws.pos_par.as<float4>() + off_disc[p];
         S.sun.exact_flat = all_exact ? 1 : 0;
         S.sun.cell_xa = all_exact ? ws.pos_xa.as<float4>() + off_disc[p] : nullptr;
         S.sun.cell_xb = all_exact ? ws.pos_xb.as<float4>() + off_disc[p] : nullptr;
         S.sun.cell_xc = all_exact ? ws.pos_xc.as<float4>() + off_disc[p] : nullptr;
-        S.sun.occ = ws.pos_occ.as<uint32_t>() + L.off_occ[p];
+        S.sun.occ = ws.pos_occ.as<uint32_t>() + (on_device ? size_t(grids[p].occ0) : L.off_occ[p]);
         S.sun.inv_cdf = hs.inv_cdf.empty() ? nullptr : ws.inv_cdf.as<double>();
         if (off_elems[p] != size_t(-1)) S.elems = ws.pos_elems.as<ElemRec>() + off_elems[p];
         S.seed = pos[p].seed;

@@ -6,6 +6,8 @@ double-precision grid probe on the same sun rays.  Both must list the same rays 
 elements, on layouts where the float test can go wrong: grids much coarser than the elements,
 kilometre-long rows (bitmaps coarser than the cells), coplanar duplicates (every ray undecided),
 elements near edge-on, narrow rotated rectangles, disabled elements, and a last tile of one ray.
+Batched runs build the same grids on the device: their positions must number the rays of single
+runs on those layouts.
 """
 import ctypes as C
 import math
@@ -52,13 +54,16 @@ def _layout(name):
             n = (math.sin(t) * math.cos(a), math.sin(t) * math.sin(a), math.cos(t))
             els.append(_elem((x, y, rng.uniform(0, 20)), n, (6.0, 3.0), zrot=rng.uniform(0, 180), enabled=k % 7 != 0))
         return els, up, 3001
+    if name == "negative":  # a negative size accepts nothing
+        e = [_elem((x, y, 0.0), up, (3.0, 3.0)) for x in range(0, 40, 5) for y in range(0, 40, 5)]
+        return e + [_elem((x, 50.0, 0.0), up, (-3.0, 3.0)) for x in range(0, 40, 5)], up, 3000
     if name == "narrow":
         return [_elem((x, y, rng.uniform(0, 5)), up + rng.normal(0, 0.4, 3), (12.0, 0.3), zrot=rng.uniform(0, 180))
                 for x, y in rng.uniform(-50, 50, (200, 2))], np.array([0.3, 0.4, math.sqrt(0.75)]), 4097
     return [_elem((x, y, 0.0), up, (1.0, 1.0)) for x in (0, 2) for y in (0, 2)], up, 1  # "four"
 
 
-@pytest.mark.parametrize("name", ["sparse", "row", "duplicates", "edge-on", "narrow", "four"])
+@pytest.mark.parametrize("name", ["sparse", "row", "duplicates", "edge-on", "narrow", "four", "negative"])
 def test_flat_probe_lists_the_general_probes_hits(product, name):
     import torch
 
@@ -88,5 +93,27 @@ def test_flat_probe_lists_the_general_probes_hits(product, name):
         got_sid, got_el = np.concatenate(got_sid), np.concatenate(got_el)
         assert len(got_sid) == hits and got_sid[-1] == nsun - 1
         assert np.array_equal(got_el + 1, first)
+    finally:
+        product.st_free_context(ctx)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("name", ["sparse", "row", "duplicates", "edge-on", "narrow", "four", "negative"])
+def test_batched_grids_number_the_single_runs_rays(product, name, prec):
+    from soltrace_b200 import scenes
+    els, sun, hits = _layout(name)
+    suns = [1e4 * np.asarray(sun), 1e4 * np.asarray([0.2, -0.3, math.sqrt(1 - 0.13)]), 1e4 * np.asarray([0.0, 0.8, 0.6])]
+    ctx = product.st_create_context()
+    try:
+        scenes.push(product, ctx, _scene(els, sun, hits))
+        product.st_b200_set_precision(ctx, prec)
+        product.st_b200_set_records(ctx, 0)
+        assert product.run_batch(ctx, 5, suns, [hits] * 3) == 1, product.messages(ctx)
+        got = [(product.batch_stats(ctx, k)["sun_rays"], product.batch_absorbed(ctx, k, 1, len(els))) for k in range(3)]
+        for k, (n, absorbed) in enumerate(got):
+            product.st_sun_xyz(ctx, *map(float, suns[k]))
+            assert product.run(ctx, 5 + k) >= 0, product.messages(ctx)
+            assert product.stats(ctx)["sun_rays"] == n
+            assert np.array_equal(product.element_counts(ctx, 1, len(els))[1], absorbed)
     finally:
         product.st_free_context(ctx)
