@@ -115,6 +115,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         : "memory");
 }
 
+// one thread of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
@@ -738,15 +749,18 @@ __global__ void k_to_bf16(long long n, const float *x, __nv_bfloat16 *y) {
 //     their group's sums;
 //   warp 8, one thread (loader): issues the weight stages, kRing ahead of their use, across
 //     layers and tiles (the next layer's weights arrive while the epilogue runs);
-//   warp 9, one thread (MMA issuer): per stage waits for its weights and for the 64-wide slice of
-//     X they multiply, issues the tcgen05.mma (128 x 256 x 16 each) and commits the stage back
-//     to the loader; the accumulator's commit wakes the epilogue.
+//   warp 9 (MMA issuer): per stage waits for its weights and for the 64-wide slice of X they
+//     multiply; one elected thread issues the tcgen05.mma (128 x 256 x 16 each) and commits the
+//     stage back to the loader; the accumulator's commit wakes the epilogue.  The whole warp runs
+//     the loop and only offsets are added to ready descriptors: with a loop that only lane 0
+//     entered and descriptors built per product, 128,000 rows took 206 us a pass and take 182
+//     here, 128 rows 31.5 and 27.6.
 // Two accumulators (2 x 256 tensor-memory columns) alternate between units (a layer, or a
 // 256-wide chunk of the output layer), so a layer's products start on the first slice of X while
 // the epilogue still writes the others, and an output chunk's epilogue overlaps the next
 // chunk's products.  With four epilogue warps and one barrier for the whole of X the tensor
 // cores waited for the epilogue of every hidden layer: 64 x 2,000 rows of the 6-layer network
-// took 338 us there and take 212 here.  Every wait is bounded; one that runs out sets the error
+// took 338 us there and take 187 here.  Every wait is bounded; one that runs out sets the error
 // flag and a shared abort flag that ends every role's loop, and the CTA drains its own copies and
 // products before freeing tensor memory.
 constexpr int kWidth = 256;                       // hidden width: the MMA N and the next layer's K
@@ -848,48 +862,57 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
             issued_sh = q;
         }
     } else if (warp == 9) {
-        // ---- MMA issuer ----
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(kWidth);
-            unsigned q = 0, u = 0, x0 = 0, x1 = 0;  // x0, x1: phases of slice 0 (a layer each) and of the others
-            bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                for (int l = 0; l < L && ok; ++l) {
-                    const int chunks = (l == L - 1) ? NC : 1;
-                    const int nst = (l == 0) ? 1 : kWidth / kBK;
-                    for (int c = 0; c < chunks && ok; ++c, ++u) {
-                        const int b = u & 1;
-                        if (u >= 2 && !mbar_wait_or_abort(&acc_free[b], ((u >> 1) - 1) & 1u, &abort_flag)) {
+        // ---- MMA issuer: the warp runs the loop (votes keep it uniform), one thread issues ----
+        constexpr uint32_t idesc = instr_desc(kWidth);
+        const bool leader = elect_one();
+        const uint64_t x_desc = smem_desc(smem_u32(X), 2048, 128), w_desc = smem_desc(smem_u32(ring), 4096, 128);
+        unsigned q = 0, slot = 0, wrap = 0, u = 0, x0 = 0, x1 = 0;  // x0, x1: phases of slice 0 (a layer each) and of the others
+        bool ok = true;
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            for (int l = 0; l < L && ok; ++l) {
+                const int chunks = (l == L - 1) ? NC : 1;
+                const int nst = (l == 0) ? 1 : kWidth / kBK;
+                for (int c = 0; c < chunks && ok; ++c, ++u) {
+                    const int b = u & 1;
+                    if (u >= 2 && !__all_sync(0xffffffffu, mbar_wait_or_abort(&acc_free[b], ((u >> 1) - 1) & 1u, &abort_flag))) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t acc = tmem + uint32_t(b * kWidth);
+                    for (int s = 0; s < nst; ++s) {
+                        if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&full[slot], wrap, &abort_flag)) ||
+                            (c == 0 && !__all_sync(0xffffffffu, mbar_wait_or_abort(&x_ready[s], (s ? x1 : x0) & 1u, &abort_flag)))) {
                             ok = false;
                             break;
                         }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        for (int s = 0; s < nst; ++s, ++q) {
-                            const int slot = q % kRing;
-                            if (!mbar_wait_or_abort(&full[slot], (q / kRing) & 1u, &abort_flag) ||
-                                (c == 0 && !mbar_wait_or_abort(&x_ready[s], (s ? x1 : x0) & 1u, &abort_flag))) {
-                                ok = false;
-                                break;
-                            }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t wb = smem_u32(ring + slot * kStageBytes);
-                            const int steps = (l == 0) ? 1 : kBK / 16;
-                            for (int j = 0; j < steps; ++j) {
-                                // X: K chunk kc at kc * 2048 (16 row groups of 128 B); weight block: K
-                                // chunk at kc * 4096 (32 row groups); a K = 16 step spans two chunks
-                                const int kstep = s * (kBK / 16) + j;
-                                const uint64_t ad = smem_desc(smem_u32(X) + uint32_t(kstep * 2 * 2048), 2048, 128);
-                                const uint64_t bd = smem_desc(wb + uint32_t(j * 2 * 4096), 4096, 128);
-                                mma_bf16(tmem + uint32_t(b * kWidth), ad, bd, idesc, (s > 0 || j > 0) ? 1u : 0u);
+                        // X: a K chunk of eight every 2048 bytes (16 row groups of 128 B); weight
+                        // block: every 4096 (32 row groups); a K = 16 step spans two chunks
+                        const uint64_t ad = x_desc + uint64_t(s * (kBK / 8 * 2048 >> 4)), bd = w_desc + uint64_t(slot * (kStageBytes >> 4));
+                        if (leader) {
+                            mma_bf16(acc, ad, bd, idesc, s > 0 ? 1u : 0u);
+                            if (l > 0) {
+#pragma unroll
+                                for (int j = 1; j < kBK / 16; ++j)
+                                    mma_bf16(acc, ad + uint64_t(j * (2 * 2048 >> 4)), bd + uint64_t(j * (2 * 4096 >> 4)), idesc, 1u);
                             }
                             mma_commit(&empty[slot]);
                         }
-                        if (ok) mma_commit(&acc_full[b]);
+                        ++q;
+                        if (++slot == kRing) {
+                            slot = 0;
+                            wrap ^= 1u;
+                        }
                     }
-                    ++x0;
-                    if (l > 0) ++x1;
+                    if (ok && leader) mma_commit(&acc_full[b]);
                 }
+                ++x0;
+                if (l > 0) ++x1;
             }
+        }
+        __syncwarp();
+        if (leader) {
             if (!ok) abort_flag = 1;
             consumed_sh = q;
             // every product this thread issued has finished before the CTA frees its memory
