@@ -745,8 +745,9 @@ __global__ void k_to_bf16(long long n, const float *x, __nv_bfloat16 *y) {
 //   warps 0-7 (epilogue): load the tile's inputs into X; per layer read the accumulator back
 //     64 columns at a time (warp w owns tensor-memory lanes 32 (w % 4) .. + 31, thread = row,
 //     and half of the 64 columns), add the bias, ReLU, round to bf16 and write that slice of X for
-//     the next layer; on the output layer apply scale/clamp and write the rows or add them into
-//     their group's sums;
+//     the next layer; on the output layer apply scale/clamp and write the rows, or, for group
+//     sums, whose products run transposed (W X^T: lane = output, column = row), add up its
+//     output's rows in registers, 32 at a time, and add once per group to the sums;
 //   warp 8, one thread (loader): issues the weight stages, kRing ahead of their use, across
 //     layers and tiles (the next layer's weights arrive while the epilogue runs);
 //   warp 9 (MMA issuer): per stage waits for its weights and for the 64-wide slice of X they
@@ -760,9 +761,12 @@ __global__ void k_to_bf16(long long n, const float *x, __nv_bfloat16 *y) {
 // the epilogue still writes the others, and an output chunk's epilogue overlaps the next
 // chunk's products.  With four epilogue warps and one barrier for the whole of X the tensor
 // cores waited for the epilogue of every hidden layer: 64 x 2,000 rows of the 6-layer network
-// took 338 us there and take 187 here.  Every wait is bounded; one that runs out sets the error
-// flag and a shared abort flag that ends every role's loop, and the CTA drains its own copies and
-// products before freeing tensor memory.
+// took 338 us there.  With the group sums' products transposed they take 137 us: summing each
+// column over rows by shuffles between lanes held the output layer up (187 us; on the device
+// 128,000 rows in groups of 2,000 182 -> 129 us, 2,000 rows 28.7 -> 23.2, 128,000 rows in groups of
+// 31, whose rows were added one atomic each, 1,179 -> 236).  Every wait is bounded; one that runs
+// out sets the error flag and a shared abort flag that ends every role's loop, and the CTA drains
+// its own copies and products before freeing tensor memory.
 constexpr int kWidth = 256;                       // hidden width: the MMA N and the next layer's K
 constexpr int kRing = 4;                          // weight stages in flight
 constexpr int kStageBytes = kWidth * kBK * 2;     // 32 KB: a 256 x 64 weight block
@@ -891,11 +895,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                         // block: every 4096 (32 row groups); a K = 16 step spans two chunks
                         const uint64_t ad = x_desc + uint64_t(s * (kBK / 8 * 2048 >> 4)), bd = w_desc + uint64_t(slot * (kStageBytes >> 4));
                         if (leader) {
-                            mma_bf16(acc, ad, bd, idesc, s > 0 ? 1u : 0u);
-                            if (l > 0) {
+                            if (l == L - 1 && g.mode == 1) {  // W X^T, 128 outputs (2048 bytes of a chunk) a half
+                                constexpr uint32_t tdesc = instr_desc(kBM);
 #pragma unroll
-                                for (int j = 1; j < kBK / 16; ++j)
-                                    mma_bf16(acc, ad + uint64_t(j * (2 * 2048 >> 4)), bd + uint64_t(j * (2 * 4096 >> 4)), idesc, 1u);
+                                for (int j = 0; j < kBK / 16; ++j)
+#pragma unroll
+                                    for (int h = 0; h < 2; ++h)
+                                        mma_bf16(acc + uint32_t(h * kBM), bd + uint64_t((j * 2 * 4096 + h * 2048) >> 4),
+                                                 ad + uint64_t(j * (2 * 2048 >> 4)), tdesc, (s > 0 || j > 0) ? 1u : 0u);
+                            } else {
+                                mma_bf16(acc, ad, bd, idesc, s > 0 ? 1u : 0u);
+                                if (l > 0) {
+#pragma unroll
+                                    for (int j = 1; j < kBK / 16; ++j)
+                                        mma_bf16(acc, ad + uint64_t(j * (2 * 2048 >> 4)), bd + uint64_t(j * (2 * 4096 >> 4)), idesc,
+                                                 1u);
+                                }
                             }
                             mma_commit(&empty[slot]);
                         }
@@ -977,61 +992,67 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs g) {
                             }
                             mbar_arrive(&x_ready[s]);
                         }
+                    } else if (g.mode == 1) {
+                        // thread = output column, accumulator column = row: the sum over the tile's rows
+                        // stays in the thread, one atomic per group that the tile meets
+                        const int n = c * kWidth + half * kBM + r;
+                        const float bn = bias_sh[l * kWidth + n];
+                        const int rows = min(kBM, g.M - t * kBM);
+                        int grp = t * kBM / g.group_rows;
+                        int left = int(min((long long)kBM, (grp + 1LL) * g.group_rows - t * kBM));  // its rows ahead
+                        float sum = 0.f;
+                        auto next_group = [&]() {
+                            atomicAdd(g.out + (long long)grp * g.n_out + n, sum);
+                            sum = 0.f;
+                            ++grp;
+                            left = min(kBM, g.group_rows);
+                        };
+                        for (int r0 = 0; r0 < rows; r0 += 32) {
+                            if (left == 0) next_group();
+                            float v[32];
+                            tmem_ld32(ta + uint32_t(half * kBM + r0), v);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                v[i] = (v[i] + bn) * g.scale;
+                                if (g.clamp) v[i] = fmaxf(v[i], 0.f);
+                            }
+                            if (left >= 32 && rows - r0 >= 32) {
+#pragma unroll
+                                for (int w = 16; w >= 1; w >>= 1)
+#pragma unroll
+                                    for (int i = 0; i < w; ++i) v[i] += v[i + w];
+                                sum += v[0];
+                                left -= 32;
+                                continue;
+                            }
+                            // rows to the end of the group, then the next groups'
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                if (r0 + i >= rows) break;
+                                if (left == 0) next_group();
+                                sum += v[i];
+                                --left;
+                            }
+                        }
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&acc_free[b]);
+                        atomicAdd(g.out + (long long)grp * g.n_out + n, sum);
                     } else {
-                        const int n0 = c * kWidth;
                         const bool valid = row < g.M;
-                        const long long grp = (long long)(valid ? row : g.M - 1) / (g.mode == 1 ? g.group_rows : 1);
-                        const long long grp0 = __shfl_sync(0xffffffffu, grp, 0);
-                        const bool uniform = __all_sync(0xffffffffu, grp0 == grp) && g.mode == 1;
                         for (int s = 0; s < kSlices; ++s) {
-                            float w32[32];
-                            tmem_ld32(ta + uint32_t(s * kBK + half * 32), w32);
+                            const int c0 = s * kBK + half * 32;
+                            float v[32];
+                            tmem_ld32(ta + uint32_t(c0), v);
+                            if (valid) {
+                                float4 *o = reinterpret_cast<float4 *>(g.out + (long long)row * g.n_out + c * kWidth + c0);
 #pragma unroll
-                            for (int q = 0; q < 2; ++q) {
-                                float *v = w32 + 16 * q;
-                                const int c0 = s * kBK + half * 32 + 16 * q;
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
+                                for (int i = 0; i < 8; ++i) {
                                     const float4 bb = bias[c0 / 4 + i];
-                                    v[4 * i] += bb.x;
-                                    v[4 * i + 1] += bb.y;
-                                    v[4 * i + 2] += bb.z;
-                                    v[4 * i + 3] += bb.w;
-                                }
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) {
-                                    float y = v[i] * g.scale;
-                                    if (g.clamp) y = fmaxf(y, 0.f);
-                                    v[i] = valid ? y : 0.f;
-                                }
-                                const int col = n0 + c0;
-                                if (g.mode == 0) {
-                                    if (valid) {
-                                        float4 *o = reinterpret_cast<float4 *>(g.out + (long long)row * g.n_out + col);
-#pragma unroll
-                                        for (int i = 0; i < 4; ++i)
-                                            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                                    }
-                                } else if (uniform) {
-                                    // the warp's 32 rows share a group: halve the 16 columns' sums across
-                                    // lanes (16 shuffles), then one atomic per column
-#pragma unroll
-                                    for (int d = 16, w = 8; d >= 2; d >>= 1, w >>= 1) {
-#pragma unroll
-                                        for (int i = 0; i < w; ++i) {
-                                            const bool hi = (lane & d) != 0;
-                                            const float send = hi ? v[i] : v[i + w];
-                                            const float keep = hi ? v[i + w] : v[i];
-                                            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-                                        }
-                                    }
-                                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                                    const int k = ((lane & 16) ? 8 : 0) + ((lane & 8) ? 4 : 0) + ((lane & 4) ? 2 : 0) +
-                                                  ((lane & 2) ? 1 : 0);
-                                    if ((lane & 1) == 0) atomicAdd(g.out + grp * g.n_out + col + k, v[0]);
-                                } else if (valid) {
-#pragma unroll
-                                    for (int i = 0; i < 16; ++i) atomicAdd(g.out + grp * g.n_out + col + i, v[i]);
+                                    float4 y = make_float4((v[4 * i] + bb.x) * g.scale, (v[4 * i + 1] + bb.y) * g.scale,
+                                                           (v[4 * i + 2] + bb.z) * g.scale, (v[4 * i + 3] + bb.w) * g.scale);
+                                    if (g.clamp)
+                                        y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
+                                    o[i] = y;
                                 }
                             }
                         }
