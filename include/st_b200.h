@@ -18,11 +18,13 @@ extern "C" {
 
 /* Arithmetic of the per-ray work.
  *   ST_B200_FP64  (default): every ray computation in double precision, rounded as the
- *                  reference's x86-64 build rounds it (no fused multiply-add).
+ *                  reference's x86-64 build rounds it (no fused multiply-add), but for the
+ *                  first-stage probe of flat rectangles, which decides hits in float
+ *                  outside float's rounding margins and the rest in double (the hits are
+ *                  the double search's).
  *   ST_B200_MIXED: aperture tests, property tables, Fresnel coefficients, error sampling
  *                  and flux binning in float; the first-stage probe of flat rectangles
- *                  decides hits in float and defers to double within float rounding (the
- *                  hits are the FP64 probe's); transforms, closed-form roots, the torus
+ *                  as above; transforms, closed-form roots, the torus
  *                  quartic, Newton refinement, reflection and refraction directions and
  *                  all counters in double / 64-bit integers (positions of explicit rays
  *                  agree with FP64 within 1e-5 m on km paths). */
@@ -193,9 +195,9 @@ int st_b200_set_ranks(st_context_t pcxt, int rank, int nranks, st_b200_allgather
  * stage aimed for sun k).  Precision and flux maps (st_b200_add_flux_map, kept per position)
  * come from the context; records are not built.  The host reads the positions' progress
  * once per wave (a few times per call), not once per position.  Positions go to the device
- * in chunks of 64 through two page-locked staging areas that the context keeps (each sized
- * for its largest chunk: a chunk is staged while the previous one runs) until
- * st_free_context.  Returns 1, or -1 with the reason in st_message(). */
+ * in chunks of 64.  First stages of flat rectangles have their sun-plane grids built on the
+ * device; others are staged, a chunk while the previous one runs, through two page-locked
+ * areas that the context keeps (each sized for its largest chunk) until st_free_context.  Returns 1, or -1 with the reason in st_message(). */
 int st_b200_sim_run_batch(st_context_t pcxt, unsigned int seed, int n_positions, const double *sun_xyz,
                           const st_uint_t *hits, const double *track_target);
 /* Results of the last batched run.  position >= 0: that position's SunRayCount, hits, stage

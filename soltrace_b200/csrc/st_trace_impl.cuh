@@ -1,16 +1,17 @@
 // Trace kernels of the B200 SolTrace path.
 //
 // A run is a sequence of sun-ray batches.  Per batch:
-//   k_probe   one thread per sun ray: generate it (generateray.cpp:58-161), find the
-//             nearest first-stage element it hits (raytrace.cpp:653-770), write the
-//             element (0 = miss) per ray and a per-block hit count;
-//   k_offsets single block: exclusive scan of the block counts;
-//   k_compact one thread per sun ray: ordered list of the rays that hit (their sun
-//             index and element), i.e. the reference's ray numbering, in which only
+//   probe     generate each sun ray (generateray.cpp:58-161) and find the nearest first-stage
+//             element it hits (raytrace.cpp:653-770): k_sun_probe_flat (first stages of flat
+//             rectangles), k_sun_candidates + k_sun_resolve (others with a sun-plane grid) or
+//             k_probe (one thread per ray); a list of the rays tested, a hit-mask bit per ray
+//             and a hit count per kProbeBlock rays;
+//   order     scan of the counts and a counting sort of the list by element; each hit gets its
+//             rank in sun-ray order, i.e. the reference's ray numbering, in which only
 //             first-stage hits consume a number (raytrace.cpp:780-798);
-//   k_trace   one thread per numbered ray: the rest of the per-ray state machine of
-//             raytrace.cpp:582-1040 through every stage, writing records, flux bins
-//             and counters.
+//   trace     the rest of the per-ray state machine of raytrace.cpp:582-1040 through every
+//             stage, writing records, flux bins and counters: k_wf_first, rounds of k_wf_search
+//             and k_wf_shade over device queues, k_wf_finish.
 // Splitting off the probe keeps the trace kernel's warps full: the sun rays that
 // miss everything (most of them on a heliostat field) never enter it.
 #pragma once
