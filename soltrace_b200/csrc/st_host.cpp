@@ -1367,19 +1367,21 @@ bool sun_setup(Context *cx, HostScene &hs) {
                     ecy[j] = c2[1];
                     xb[j] = float4{0.f, 0.f, 0.f, 0.f};
                     if (never(e)) continue;
-                    if (!(fabs(det) > 1e-3 * la * lb) || !(fabs(n2[2]) > 1e-3)) {
-                        xc[j] = float4{0.f, 0.f, 0.f, INFINITY};  // near edge-on: always decided in double
+                    // margins over the cells the element is listed in, |q| <= Q there: the float
+                    // rounding of (u, v) and of the depth, and the coordinates' own error
+                    const double gx = -n2[0] / n2[2], gy = -n2[1] / n2[2];
+                    const double Q = disc[j].z + 1.5 * cell, err = fp.eps * (1.0 + fabs(gx) + fabs(gy));
+                    const double tol = 1e-6 * (fabs(c2[2]) + (fabs(gx) + fabs(gy)) * Q) + err + 1e-5;
+                    if (!(fabs(det) > 1e-3 * la * lb) || !(fabs(n2[2]) > 1e-3) ||
+                        !before_start_plane(c2[2] - fabs(a2[2]) - fabs(b2[2]), tol)) {
+                        xc[j] = float4{0.f, 0.f, 0.f, INFINITY};  // always decided in double
                         occ.mark_disc(c2[0] - sun.xmin, c2[1] - sun.ymin, disc[j].z + 2.0 * fp.eps);
                     } else {
                         const double i4[4] = {b2[1] / det, -b2[0] / det, -a2[1] / det, a2[0] / det};
-                        const double gx = -n2[0] / n2[2], gy = -n2[1] / n2[2];
-                        // margins over the cells the element is listed in, |q| <= Q there: the float
-                        // rounding of (u, v) and of the depth, and the coordinates' own error
-                        const double Q = disc[j].z + 1.5 * cell, err = fp.eps * (1.0 + fabs(gx) + fabs(gy));
                         const double row = std::max(fabs(i4[0]) + fabs(i4[1]), fabs(i4[2]) + fabs(i4[3]));
                         xb[j] = float4{float(i4[0]), float(i4[1]), float(i4[2]), float(i4[3])};
                         xc[j] = float4{float(gx), float(gy), float(c2[2]), float((6e-7 * Q + err) * row + 1e-6)};
-                        xtol[j] = float(1e-6 * (fabs(c2[2]) + (fabs(gx) + fabs(gy)) * Q) + err + 1e-5);
+                        xtol[j] = float(tol);
                         occ.mark(c2[0] - sun.xmin, c2[1] - sun.ymin, fabs(a2[0]) + fabs(b2[0]),
                                  fabs(a2[1]) + fabs(b2[1]), i4);
                     }

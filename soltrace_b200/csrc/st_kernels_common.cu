@@ -238,18 +238,19 @@ __global__ void __launch_bounds__(128) k_pos_footprints(const PosGridBuild b) {
                     atomicOr(&b.occ[g.occ0 + uint32_t(iy) * uint32_t(g.ostride) + uint32_t(ix >> 5)], 1u << (ix & 31));
                 }
         };
-        if (!flat_on || !(fabs(n[2]) > 1e-3)) {
-            f.xc = make_float4(0.f, 0.f, 0.f, INFINITY);  // near edge-on: always decided in double
+        const double gx = -n[0] / n[2], gy = -n[1] / n[2];
+        const double Q = f.disc.z + 1.5 * g.cell, err = g.eps * (1.0 + fabs(gx) + fabs(gy));
+        const double tol = 1e-6 * (fabs(c[2]) + (fabs(gx) + fabs(gy)) * Q) + err + 1e-5;
+        if (!flat_on || !(fabs(n[2]) > 1e-3) || !before_start_plane(c[2] - hx * fabs(a[2]) - hy * fabs(bb[2]), tol)) {
+            f.xc = make_float4(0.f, 0.f, 0.f, INFINITY);  // always decided in double
             const double r = f.disc.z + 2.0 * g.eps + g.pad;
             mark(r, r, nullptr);
         } else {
             const double i4[4] = {bb[1] / (d1 * hx), -bb[0] / (d1 * hx), -a[1] / (d1 * hy), a[0] / (d1 * hy)};
-            const double gx = -n[0] / n[2], gy = -n[1] / n[2];
-            const double Q = f.disc.z + 1.5 * g.cell, err = g.eps * (1.0 + fabs(gx) + fabs(gy));
             const double row = fmax(fabs(i4[0]) + fabs(i4[1]), fabs(i4[2]) + fabs(i4[3]));
             f.xb = make_float4(float(i4[0]), float(i4[1]), float(i4[2]), float(i4[3]));
             f.xc = make_float4(float(gx), float(gy), float(c[2]), float((6e-7 * Q + err) * row + 1e-6));
-            f.xtol = float(1e-6 * (fabs(c[2]) + (fabs(gx) + fabs(gy)) * Q) + err + 1e-5);
+            f.xtol = float(tol);
             mark((hx * fabs(a[0]) + hy * fabs(bb[0])) * (1.0 + 1e-5) + g.pad,
                  (hx * fabs(a[1]) + hy * fabs(bb[1])) * (1.0 + 1e-5) + g.pad, i4);
         }

@@ -24,6 +24,7 @@ constexpr int kMaxFluxMaps = 8;
 constexpr int kSunCdfCells = 4096;
 constexpr int kSunInvCells = 8192;
 constexpr int kMaxOccWords = 16384;  // occupancy bitmap of the sun-plane grid: at most 64 KB
+constexpr double kSunRayStart = -10000.0;  // sun-frame z that generated sun rays start from
 
 // surface model codes after coretrace/input.cpp:288-366 translation
 enum SurfType : int {
@@ -156,8 +157,8 @@ struct SunDev {
     // first stages of flat rectangles only (exact_flat), per cell entry: the footprint centre
     // relative to the cell's lower corner, the depth's margin and the element (xa); the exact
     // footprint's dual basis rows, unpadded (xb); the depth slopes along the sun's z, the depth at
-    // the centre and the margin of the footprint test (xc; +inf: no exact footprint, always
-    // decided in double)
+    // the centre and the margin of the footprint test (xc; +inf: always decided in double, as an
+    // element near edge-on or reaching behind the rays' starting plane)
     int exact_flat;
     float fcell;                    // gcell
     // sun-plane point in fixed point: with U the top 32 bits of a coordinate's uniform variate,
@@ -173,6 +174,14 @@ struct SunDev {
     const float4 *cell_xb;          // i00, i01, i10, i11
     const float4 *cell_xc;          // dz/dx, dz/dy, z at the centre, footprint margin
 };
+
+// Whether a flat element whose smallest depth along the sun's z is `low`, known to within `tol`,
+// lies wholly ahead of the rays' starting plane.  The element test moves a ray 1e-5 m along itself
+// and refuses hits behind it, which the probe's float test (footprint and depth order) does not
+// look at; other elements are left to the double search.
+__host__ __device__ inline bool before_start_plane(double low, double tol) {
+    return low - tol > kSunRayStart + 2e-5;
+}
 
 struct SceneDev {
     const ElemRec *elems;

@@ -51,7 +51,7 @@ __device__ __forceinline__ void make_ray(const SceneDev &S, uint64_t sid, RayRng
     }
     xs = sun.xmin + (sun.xmax - sun.xmin) * rng.u();
     ys = sun.ymin + (sun.ymax - sun.ymin) * rng.u();
-    const double psun[3] = {xs, ys, -10000.0}, csun[3] = {0.0, 0.0, 1.0};
+    const double psun[3] = {xs, ys, kSunRayStart}, csun[3] = {0.0, 0.0, 1.0};
     double pst[3], cst[3];
     to_ref(sun.Rsun, sun.pos_sun_stage, psun, csun, pst, cst);
     to_ref(S.stages[0].R, S.stages[0].o, pst, cst, pg, cg);
@@ -281,7 +281,7 @@ __device__ __forceinline__ int nearest_kind(const SceneDev &S, const StageRec &s
 __device__ __forceinline__ void sun_ray_in_stage(const SceneDev &S, double xs, double ys, double ps[3], double cs[3]) {
     const SunDev &sun = S.sun;
     const StageRec &st = S.stages[0];
-    const double psun[3] = {xs, ys, -10000.0}, csun[3] = {0.0, 0.0, 1.0};
+    const double psun[3] = {xs, ys, kSunRayStart}, csun[3] = {0.0, 0.0, 1.0};
     double pst[3], cst[3], pg[3], cg[3];
     to_ref(sun.Rsun, sun.pos_sun_stage, psun, csun, pst, cst);
     to_ref(st.R, st.o, pst, cst, pg, cg);
