@@ -17,6 +17,7 @@
 
 #include "st_host.h"
 #include "st_launch.h"
+#include "st_room.h"
 
 namespace stb {
 
@@ -571,18 +572,11 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     CK(d_ecount.ensure(size_t(n_elem0) * 4));
     CK(d_ecursor.ensure(size_t(n_elem0) * 4));
     CK(d_etotal.ensure(8));
-    unsigned long long rec_cap = 0, save_cap = 0;
+    RecordRoom<DevBuf> rec(d_recs, sizeof(RecordDev));
+    unsigned long long save_cap = 0;
     (void)dev_sms;
     out.setup_ms = ms_since(t_setup);
 
-    // room for `need` records in the run's record buffer, keeping the first `keep`
-    auto rec_room = [&](unsigned long long need, unsigned long long keep) -> cudaError_t {
-        if (need <= rec_cap) return cudaSuccess;
-        const unsigned long long cap = std::max(need, rec_cap + rec_cap / 2);
-        cudaError_t e = d_recs.grow_keep(cap * sizeof(RecordDev), keep * sizeof(RecordDev), st);
-        if (e == cudaSuccess) rec_cap = cap;
-        return e;
-    };
     double rec_per_ray = 2.0 * nst;  // records per numbered ray expected when sizing the buffer
     for (int attempt = 0; attempt < 4; ++attempt) {
         bool restart = false;
@@ -601,8 +595,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         const unsigned long long n_pre = rq.pre_records.size();
         unsigned long long nrec_run = 0;  // records written so far (read after every batch)
         if (rq.records) {
-            CK(d_recs.ensure(std::max<unsigned long long>(rec_cap, n_pre + 4096) * sizeof(RecordDev)));
-            rec_cap = d_recs.bytes / sizeof(RecordDev);
+            CK(rec.begin(n_pre + 4096));
             if (n_pre)
                 CK(cudaMemcpyAsync(d_recs.p, rq.pre_records.data(), n_pre * sizeof(RecordDev),
                                    cudaMemcpyHostToDevice, st));
@@ -735,9 +728,9 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             const uint64_t n1 = rq.replay_rows.size() / 7;
             CK(upload(ws.replay_rows, rq.replay_rows, st, out.h2d_bytes));
             CK(upload(ws.replay_fe0, rq.replay_fe0, st, out.h2d_bytes));
-            if (rq.records) CK(rec_room(nrec_run + std::max<uint64_t>(n1, 1) * uint64_t(nst) * 2 + 4096, nrec_run));
+            if (rq.records) CK(rec.room(nrec_run + std::max<uint64_t>(n1, 1) * uint64_t(nst) * 2 + 4096, nrec_run, st));
             O.recs = rq.records ? d_recs.as<RecordDev>() : nullptr;
-            O.rec_cap = rq.records ? rec_cap : 0;
+            O.rec_cap = rq.records ? rec.cap : 0;
             WfState W;
             WfQueues Q;
             CK(wf_buffers(ws, S, n1, W, Q));
@@ -760,10 +753,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             out.batches = 1;
             CK(read_back());
             const unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
-            if (rq.records && nrec > rec_cap) {
-                rec_cap = nrec + nrec / 4 + 4096;
-                continue;
-            }
+            if (rq.records && rec.overflowed(rec.report(nrec).data(), 1)) continue;
             bool save_over = false;
             CK(save_collect(save_over));
             if (save_over) continue;
@@ -829,10 +819,10 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                     const uint64_t numbered = multi ? global_done : rs.hits_done;
                     const uint64_t left = explicit_mode ? n : rq.n_hits - std::min<uint64_t>(rq.n_hits, numbered);
                     const double est = double(std::min<uint64_t>(n, left)) * rec_per_ray;
-                    CK(rec_room(nrec_run + uint64_t(est) + 4096, nrec_run));
+                    CK(rec.room(nrec_run + uint64_t(est) + 4096, nrec_run, st));
                 }
                 O.recs = rq.records ? d_recs.as<RecordDev>() : nullptr;
-                O.rec_cap = rq.records ? rec_cap : 0;
+                O.rec_cap = rq.records ? rec.cap : 0;
                 cudaEvent_t p0 = new_event(), p1 = new_event(), p2 = new_event();
                 CK(cudaEventRecord(p0, st));
                 if (n > 0) {
@@ -917,23 +907,15 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 if (sync_each) {
                     CK(read_back());
                     rs = ws.mail->rs;
-                    unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
-                    const unsigned long long nrec_local = nrec;
-                    bool overflow = rq.records && nrec > rec_cap;
-                    if (multi) {  // a rank out of record room makes every rank re-run, in step
-                        std::vector<unsigned long long> got;
-                        if (!exchange({overflow ? 1ull : 0ull, rec_cap, nrec}, got)) {
-                            out.error = "the exchange of record counts between ranks failed";
-                            return false;
-                        }
-                        for (int k = 0; k < R; ++k) {
-                            overflow = overflow || got[3 * size_t(k)] != 0;
-                            rec_cap = std::max<unsigned long long>(rec_cap, got[3 * size_t(k) + 1]);
-                            nrec = std::max<unsigned long long>(nrec, got[3 * size_t(k) + 2]);
-                        }
+                    const unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
+                    const auto report = rec.report(nrec);
+                    std::vector<unsigned long long> reports(report.begin(), report.end());
+                    if (multi && !exchange({report[0], report[1]}, reports)) {
+                        out.error = "the exchange of record counts between ranks failed";
+                        return false;
                     }
-                    if (overflow) {
-                        rec_cap = nrec + nrec / 4 + 4096;  // re-run the whole job with room for it
+                    // a rank out of record room makes every rank re-run the whole job, in step
+                    if (rq.records && rec.overflowed(reports.data(), R)) {
                         restart = true;
                         break;
                     }
@@ -944,7 +926,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                         break;
                     }
                     if (rq.records) {
-                        nrec_run = nrec_local;
+                        nrec_run = nrec;
                         if (!multi && rs.hits_done > 0)
                             rec_per_ray = std::max(1.0, 1.5 * double(nrec_run - n_pre) / double(rs.hits_done));
                     }
@@ -1073,7 +1055,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                     tt_drop[s] = out.max_enter[size_t(s)];
             }
             for (const RecordDev &r : rq.pre_records) rb = std::max(rb, r.raynum);
-            const std::string err = order_records(ws, d_recs.as<RecordDev>(), std::min(nrec_run, rec_cap), nst,
+            const std::string err = order_records(ws, d_recs.as<RecordDev>(), std::min(nrec_run, rec.cap), nst,
                                                   drop_later, tt_drop, rb, out.rec, out.d2h_bytes, st);
             if (!err.empty()) {
                 out.error = err;
