@@ -9,12 +9,7 @@ namespace stb {
 template <int FLAT>
 static void resolve(const SceneDev &S, uint64_t s0, const ProbeOut &o, const RunState *rs, cudaStream_t st) {
     // persistent grid: every resident block on every SM
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sun_resolve<0, kResolveMinBlocks, FLAT>, kResolveBlock,
-                                                      0);
-        per_sm = per_sm > 0 ? per_sm : 1;
-    }
+    static const int per_sm = resident_blocks(k_sun_resolve<0, kResolveMinBlocks, FLAT>, kResolveBlock);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -53,6 +53,15 @@ constexpr int kWfFirstFlatMinBlocksMixed = ST_FIRST_FLAT_MINB_MIXED;  // the sam
 constexpr int kWfClosedShadeMinBlocks = 5;
 constexpr int kWfClosedShadeMinBlocksMixed = 4;
 
+// Blocks of a kernel that an SM keeps resident (at least 1): the grids of persistent kernels.  Callers
+// keep it in a `static const`, which threads that come first together wait for.
+template <typename... A>
+inline int resident_blocks(void (*kernel)(A...), int threads) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess) n = 0;
+    return n > 0 ? n : 1;
+}
+
 enum RunFlags : unsigned {
     kFlagHitCap = 1u,         // a ray reached kMaxHitsPerStage in one stage
     kFlagBadInteraction = 2u, // interaction type other than 1 or 2 (raytrace.cpp:943-946)

@@ -1941,11 +1941,7 @@ template <int MIXED, int RECORDS, int KIND>
 static void wf_launch_search(const SceneDev &S, const TraceOut &O, const WfState &W, const WfQueues &Q, int r, int k,
                              int sms, cudaStream_t st) {
     // persistent grid: every block the kernel can keep resident on every SM
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_search<MIXED, RECORDS, KIND>, kTraceBlock, 0);
-        per_sm = per_sm > 0 ? per_sm : 1;
-    }
+    static const int per_sm = resident_blocks(k_wf_search<MIXED, RECORDS, KIND>, kTraceBlock);
     k_wf_search<MIXED, RECORDS, KIND><<<sms * per_sm, kTraceBlock, 0, st>>>(S, O, W, Q, r, k);
 }
 
@@ -1954,18 +1950,16 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
                      const uint32_t *total, const RunState *rs, const TraceOut &O, const WfState &W,
                      const WfQueues &Q, const ReplayIn *replay, cudaStream_t st) {
     // persistent grids: every block the kernels can keep resident on every SM
-    static int per_sm[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (per_sm[0] == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_wf_first<MIXED, RECORDS, 0>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[4], k_wf_first<MIXED, RECORDS, 1>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[5], k_wf_first<MIXED, RECORDS, 2>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[7], k_wf_first<MIXED, RECORDS, 3>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_wf_shade<MIXED, RECORDS, 0>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[3], k_wf_shade<MIXED, RECORDS, 1>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_wf_finish<MIXED, RECORDS, 0>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[6], k_wf_finish<MIXED, RECORDS, 1>, kTraceBlock, 0);
-        for (int &x : per_sm) x = x > 0 ? x : 1;
-    }
+    static const struct Resident {
+        int first[4], shade[2], finish[2];
+    } per_sm = {{resident_blocks(k_wf_first<MIXED, RECORDS, 0>, kTraceBlock),
+                 resident_blocks(k_wf_first<MIXED, RECORDS, 1>, kTraceBlock),
+                 resident_blocks(k_wf_first<MIXED, RECORDS, 2>, kTraceBlock),
+                 resident_blocks(k_wf_first<MIXED, RECORDS, 3>, kTraceBlock)},
+                {resident_blocks(k_wf_shade<MIXED, RECORDS, 0>, kTraceBlock),
+                 resident_blocks(k_wf_shade<MIXED, RECORDS, 1>, kTraceBlock)},
+                {resident_blocks(k_wf_finish<MIXED, RECORDS, 0>, kTraceBlock),
+                 resident_blocks(k_wf_finish<MIXED, RECORDS, 1>, kTraceBlock)}};
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1975,18 +1969,18 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
     int launches = 2;
     cudaMemsetAsync(Q.counts, 0, sizeof(uint32_t) * (R + 1) * (nq + 1), st);
     if (replay)
-        k_wf_replay<MIXED, RECORDS><<<sms * per_sm[0], kTraceBlock, 0, st>>>(S, O, W, *replay, Q);
+        k_wf_replay<MIXED, RECORDS><<<sms * per_sm.first[0], kTraceBlock, 0, st>>>(S, O, W, *replay, Q);
     else if (stage_search_kind(S.stages[0]) == kSearchFlat)  // heliostat fields: blocking search fused
-        k_wf_first<MIXED, RECORDS, 2><<<sms * per_sm[5], kTraceBlock, 0, st>>>(S, hits, total, rs,
+        k_wf_first<MIXED, RECORDS, 2><<<sms * per_sm.first[2], kTraceBlock, 0, st>>>(S, hits, total, rs,
                                                                                  O, W, Q);
     else if (S.stages[0].flat_only)  // a first stage of flat elements only
-        k_wf_first<MIXED, RECORDS, 1><<<sms * per_sm[4], kTraceBlock, 0, st>>>(S, hits, total, rs,
+        k_wf_first<MIXED, RECORDS, 1><<<sms * per_sm.first[1], kTraceBlock, 0, st>>>(S, hits, total, rs,
                                                                                  O, W, Q);
     else if (S.stages[0].closed_only)
-        k_wf_first<MIXED, RECORDS, 3><<<sms * per_sm[7], kTraceBlock, 0, st>>>(S, hits, total, rs,
+        k_wf_first<MIXED, RECORDS, 3><<<sms * per_sm.first[3], kTraceBlock, 0, st>>>(S, hits, total, rs,
                                                                                  O, W, Q);
     else
-        k_wf_first<MIXED, RECORDS, 0><<<sms * per_sm[0], kTraceBlock, 0, st>>>(S, hits, total, rs,
+        k_wf_first<MIXED, RECORDS, 0><<<sms * per_sm.first[0], kTraceBlock, 0, st>>>(S, hits, total, rs,
                                                                                  O, W, Q);
     for (int r = 0; r < R; ++r) {
         for (int k = 0; k < nq; ++k) {
@@ -2001,15 +1995,15 @@ static int wf_launch(const SceneDev &S, const HitRec *hits,
             ++launches;
         }
         if (all_closed)
-            k_wf_shade<MIXED, RECORDS, 1><<<sms * per_sm[3], kTraceBlock, 0, st>>>(S, O, W, Q, r);
+            k_wf_shade<MIXED, RECORDS, 1><<<sms * per_sm.shade[1], kTraceBlock, 0, st>>>(S, O, W, Q, r);
         else
-            k_wf_shade<MIXED, RECORDS, 0><<<sms * per_sm[1], kTraceBlock, 0, st>>>(S, O, W, Q, r);
+            k_wf_shade<MIXED, RECORDS, 0><<<sms * per_sm.shade[0], kTraceBlock, 0, st>>>(S, O, W, Q, r);
         ++launches;
     }
     if (all_closed)
-        k_wf_finish<MIXED, RECORDS, 1><<<sms * per_sm[6], kTraceBlock, 0, st>>>(S, O, W, Q);
+        k_wf_finish<MIXED, RECORDS, 1><<<sms * per_sm.finish[1], kTraceBlock, 0, st>>>(S, O, W, Q);
     else
-        k_wf_finish<MIXED, RECORDS, 0><<<sms * per_sm[2], kTraceBlock, 0, st>>>(S, O, W, Q);
+        k_wf_finish<MIXED, RECORDS, 0><<<sms * per_sm.finish[0], kTraceBlock, 0, st>>>(S, O, W, Q);
     return launches;
 }
 
