@@ -17,9 +17,15 @@ bool launch_sun_probe_flat(const SceneDev &S, uint64_t s0, uint32_t n, const Pro
     // outputs a caller without room for the undecided rays (or with one word per ray) asks for
     // come from the general grid probe
     if (!S.sun.exact_flat || !S.stages[0].flat_only || !o.amb || !o.cand_el || !o.hit_mask || o.hit_elem) return false;
-    const int smem = kFlatBlock / 32 * kFlatWarpBytes + S.sun.occ_words * int(sizeof(uint32_t));
-    if (cudaFuncSetAttribute(k_sun_probe_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    constexpr int kWarps = kFlatBlock / 32 * kFlatWarpBytes, kMost = kWarps + kMaxOccWords * int(sizeof(uint32_t));
+    if (S.sun.occ_words > kMaxOccWords) return false;
+    // the limit belongs to the kernel on its device, for every thread: always the largest bitmap's, so
+    // that a thread setting it never lowers it under another's launch
+    if (cudaFuncSetAttribute(k_sun_probe_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess) {
+        cudaGetLastError();  // not an error of the run, which takes the general grid probe
         return false;
+    }
+    const int smem = kWarps + S.sun.occ_words * int(sizeof(uint32_t));
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
