@@ -674,8 +674,8 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThread
     const bool wide = cols % 8 == 0 && (reinterpret_cast<uintptr_t>(dz) & 15) == 0;
     if (c0 < cols) {
 #pragma unroll 4
-        for (int r = int(cluster.block_rank()) * kLanes + lane; r < rows; r += kSumCluster * kLanes) {
-            const __nv_bfloat16 *p = dz + (long long)r * cols + c0;
+        for (long long r = int(cluster.block_rank()) * kLanes + lane; r < rows; r += kSumCluster * kLanes) {
+            const __nv_bfloat16 *p = dz + r * cols + c0;
             if (wide) {
                 const uint4 v = *reinterpret_cast<const uint4 *>(p);
                 const uint32_t h[4] = {v.x, v.y, v.z, v.w};
