@@ -17,6 +17,7 @@
 
 #include "st_host.h"
 #include "st_launch.h"
+#include "st_rebind.h"
 #include "st_room.h"
 
 namespace stb {
@@ -450,12 +451,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         out.error = "CUDA device ordinal out of range";
         return false;
     }
-    CK(cudaSetDevice(rq.device));
-    if (ws.device != rq.device) {  // a workspace serves one device: start afresh on another
-        ws.~Workspace();
-        new (&ws) Workspace();
-        ws.device = rq.device;
-    }
+    CK(rebind(ws, rq.device, cudaSetDevice));
     if (!ws.stream) CK(cudaStreamCreateWithFlags(&ws.stream, cudaStreamNonBlocking));
     cudaStream_t st = ws.stream;
     DevBuf &d_elems = ws.elems, &d_optics = ws.optics, &d_surf = ws.surf, &d_tables = ws.tables, &d_bvh = ws.bvh,
@@ -1131,12 +1127,7 @@ struct PosLayout {
 }  // namespace
 
 bool workspace_bind(Workspace &ws, int device) {
-    if (cudaSetDevice(device) != cudaSuccess) return false;
-    if (ws.device != device) {  // a workspace serves one device: start afresh on another
-        ws.~Workspace();
-        new (&ws) Workspace();
-        ws.device = device;
-    }
+    if (rebind(ws, device, cudaSetDevice) != cudaSuccess) return false;
     return ws.stream || cudaStreamCreateWithFlags(&ws.stream, cudaStreamNonBlocking) == cudaSuccess;
 }
 
@@ -1213,12 +1204,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
         out.ok = true;
         return true;
     }
-    CK(cudaSetDevice(rq.device));
-    if (ws.device != rq.device) {
-        ws.~Workspace();
-        new (&ws) Workspace();
-        ws.device = rq.device;
-    }
+    CK(rebind(ws, rq.device, cudaSetDevice));
     if (!ws.stream) CK(cudaStreamCreateWithFlags(&ws.stream, cudaStreamNonBlocking));
     cudaStream_t st = ws.stream;
     uint64_t &h2d = out.h2d_bytes;
