@@ -36,7 +36,7 @@ UNITS = {
     "st_stinput.cpp": [],
 }
 CLI = os.path.join(HERE, "strace_b200")  # command-line tracer (csrc/strace_main.cpp)
-HEADERS = ["st_scene.h", "st_device.cuh", "st_trace_impl.cuh", "st_host.h", "st_launch.h", "st_rebind.h", "st_room.h"]
+HEADERS = ["st_scene.h", "st_device.cuh", "st_trace_impl.cuh", "st_host.h", "st_hostblock.h", "st_launch.h", "st_rebind.h", "st_room.h"]
 
 
 def _nvcc() -> str:

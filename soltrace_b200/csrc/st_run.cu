@@ -16,6 +16,7 @@
 #include <thread>
 
 #include "st_host.h"
+#include "st_hostblock.h"
 #include "st_launch.h"
 #include "st_rebind.h"
 #include "st_room.h"
@@ -78,6 +79,15 @@ cudaError_t upload(DevBuf &b, const std::vector<T> &v, cudaStream_t s, uint64_t 
     return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
+struct PageLocked {
+    static bool alloc(void **p, size_t bytes) {
+        if (cudaMallocHost(p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
+    static void free(void *p) { cudaFreeHost(p); }
+};
+
 }  // namespace
 
 // What a batch of sun rays in flight works in: the probe's lists, the sorted hits and the trace's
@@ -137,7 +147,7 @@ struct Workspace : Scratch {
     // the scene whose tables the buffers above hold (HostScene::version), 0 for none: a run on
     // the same scene copies nothing of it again
     uint64_t scene_version = 0;
-    // page-locked landing place of what the host reads back per batch, so that one wait covers all
+    // landing place of what the host reads back per batch, so that one wait covers all
     struct Mail {
         RunState rs;
         RunCounters ctr;
@@ -146,20 +156,18 @@ struct Workspace : Scratch {
     } *mail = nullptr;
     unsigned long long *acc_host = nullptr;  // the same for accumulators of up to kAccHost values
     static constexpr size_t kAccHost = 1u << 16;
+    HostBlock<PageLocked> mail_block;
     cudaError_t mailbox() {  // one allocation: the accumulators' place follows the mail
         if (mail) return cudaSuccess;
         constexpr size_t kMail = (sizeof(Mail) + 63) / 64 * 64;
-        void *p = nullptr;
-        const cudaError_t e = cudaMallocHost(&p, kMail + kAccHost * sizeof(unsigned long long));
-        if (e == cudaSuccess) {
-            mail = static_cast<Mail *>(p);
-            acc_host = reinterpret_cast<unsigned long long *>(static_cast<char *>(p) + kMail);
-        }
-        return e;
+        char *p = static_cast<char *>(mail_block.take(kMail + kAccHost * sizeof(unsigned long long)));
+        if (!p) return cudaErrorMemoryAllocation;
+        mail = reinterpret_cast<Mail *>(p);
+        acc_host = reinterpret_cast<unsigned long long *>(p + kMail);
+        return cudaSuccess;
     }
     ~Workspace() {
         if (device >= 0) cudaSetDevice(device);
-        if (mail) cudaFreeHost(mail);
         for (int k = 0; k < 2; ++k)
             if (pos_host[k]) cudaFreeHost(pos_host[k]);
         if (rec_host) {
