@@ -104,7 +104,10 @@ struct Context {
     std::vector<std::vector<unsigned long long>> elem_first, elem_absorbed, elem_delivered;
     int (*cb)(unsigned long, unsigned long, unsigned long, unsigned long, unsigned long, void *) = nullptr;
     void *cbdata = nullptr;
-    double last_hit_rate = 0.0;  // batch planning hint carried between runs of a context
+    // batch planning hint carried between runs of a context: the last run's hits per sun ray, and the
+    // scene (HostScene::version) that it was measured on
+    double last_hit_rate = 0.0;
+    uint64_t last_hit_scene = 0;
     // stage data (st_b200_set_save_stage_data / st_b200_sim_run_replay, stapi.cpp:680-728)
     bool save_stage_data = false;
     std::vector<double> stage_s0, stage_s1;  // saved: 8 doubles per stage-1 record, 7 per ray
@@ -1711,6 +1714,7 @@ int run(Context *cx, unsigned seed) {
     rq.callback = cx->cb;
     rq.cbdata = cx->cbdata;
     rq.hit_rate_hint = cx->last_hit_rate;
+    rq.hint_of_scene = cx->last_hit_scene == hs.version;
     rq.save_stage_data = cx->save_stage_data;
     rq.rank = cx->rank;
     rq.nranks = cx->nranks;
@@ -1774,7 +1778,10 @@ int run(Context *cx, unsigned seed) {
         return -1;
     }
     cx->sun_rays = rr.sun_rays;
-    if (rr.sun_rays > 0 && cx->ex_pos.empty()) cx->last_hit_rate = double(rr.ray_hits) / double(rr.sun_rays);
+    if (rr.sun_rays > 0 && cx->ex_pos.empty()) {
+        cx->last_hit_rate = double(rr.ray_hits) / double(rr.sun_rays);
+        cx->last_hit_scene = hs.version;
+    }
     const int nst = int(cx->stages.size());
     const uint32_t N = uint32_t(rr.ray_hits);
     const bool drop_later = !cx->replaying && nst > 1 && rr.stage_entries[1] == 1 && rr.max_enter[1] == N;

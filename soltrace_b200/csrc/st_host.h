@@ -57,7 +57,8 @@ struct RunRequest {
     std::vector<FluxMapReq> flux;
     int (*callback)(unsigned long, unsigned long, unsigned long, unsigned long, unsigned long, void *) = nullptr;
     void *cbdata = nullptr;
-    double hit_rate_hint = 0.0;  // expected first-stage hits per sun ray (0 = measure with a pilot batch)
+    double hit_rate_hint = 0.0;  // the last run's first-stage hits per sun ray (0: none)
+    bool hint_of_scene = false;  // that run was on this very scene
     bool save_stage_data = false;       // keep the rays leaving stages 1 and 2 (RunResult::saved)
     bool replay = false;                // rays enter stage 2 from replay_rows instead of the sun
     std::vector<double> replay_rows;    // 7 doubles per ray: global position, direction, ray number

@@ -689,8 +689,16 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         };
         uint64_t sun_next = 0;
         uint64_t global_done = 0;  // over several ranks: hits numbered by all ranks so far
-        // hits per sun ray: the last run's, or the scene's estimate, or (0) a pilot batch's
-        double p_est = rq.hit_rate_hint > 0 ? rq.hit_rate_hint : multi ? 0.0 : hs.hit_rate / 1.05;
+        // Hits per sun ray: the last run's on this scene; else the scene's estimate, which is at least the
+        // rate, or another scene's rate where it lies within a quarter of that; else another scene's
+        // rate, for at most kForeignRays sun rays a hit until it is measured (a sparse scene's rate would
+        // queue its billions of sun rays for a dense one); else (0) a pilot batch's.
+        constexpr uint64_t kForeignRays = 16;  // twice what a heliostat field needs
+        const double scene_rate = multi ? 0.0 : hs.hit_rate / 1.05, hint = rq.hit_rate_hint;
+        const bool foreign = hint > 0 && !rq.hint_of_scene;
+        double p_est = hint > 0 ? hint : scene_rate;
+        if (foreign && scene_rate > 0 && !(hint <= scene_rate && hint >= 0.25 * scene_rate)) p_est = scene_rate;
+        bool unmeasured = foreign && !(scene_rate > 0);
         RunState rs = rs0;
         size_t ev_used = 0;
         auto new_event = [&]() {
@@ -786,6 +794,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                     want = std::min<uint64_t>(uint64_t(1) << 20, rq.max_sun - sun_next);  // pilot batch
                 else
                     want = uint64_t(1.03 * double(need) / p_est) + 65536;
+                if (unmeasured) want = std::min(want, std::max(uint64_t(1) << 20, kForeignRays * need));
+                unmeasured = false;
                 want = std::min<uint64_t>(want, rq.max_sun - sun_next);
             }
             if (want == 0) {
