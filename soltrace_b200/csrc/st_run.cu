@@ -444,6 +444,7 @@ static std::string order_records(Workspace &ws, const RecordDev *recs, unsigned 
         cudaError_t e_ = (x);                                                                 \
         if (e_ != cudaSuccess) {                                                              \
             out.error = std::string("CUDA error: ") + cudaGetErrorString(e_) + " at " #x;     \
+            cudaGetLastError(); /* not the next run's error */                                \
             return false;                                                                     \
         }                                                                                     \
     } while (0)
@@ -1090,6 +1091,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         cudaError_t e_ = (x);                                                                 \
         if (e_ != cudaSuccess) {                                                              \
             out.error = std::string("CUDA error: ") + cudaGetErrorString(e_) + " at " #x;     \
+            cudaGetLastError(); /* not the next run's error */                                \
             return false;                                                                     \
         }                                                                                     \
     } while (0)
