@@ -574,9 +574,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     // one element and walk the same candidates)
     const uint32_t n_elem0 = uint32_t(S.stages[0].n_elem);
     DevBuf &d_ecount = ws.ecount, &d_ecursor = ws.ecursor, &d_etotal = ws.etotal, &d_s_hits = ws.s_hits;
-    CK(d_ecount.ensure(size_t(n_elem0) * 4));
-    CK(d_ecursor.ensure(size_t(n_elem0) * 4));
-    CK(d_etotal.ensure(8));
     RecordRoom<DevBuf> rec(d_recs, sizeof(RecordDev));
     unsigned long long save_cap = 0;
     (void)dev_sms;
@@ -779,10 +776,16 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         // its buffers are taken with the pilot's (two sun rays a hit, at most 2^22 rays or 0.7 GB),
         // as growing them later frees and allocates some twenty: the second run of 1e6 hits of the
         // dish took 10.4 ms, and takes 0.64 with the room there.  Runs of more hits grow them for
-        // their own second batch.  Where the room is not to be had, the batches ask for what they need.
+        // their own second batch.  Where the room is not to be had, all of it is given back and the batches
+        // ask for what they need.
         if (!explicit_mode && !rq.replay && !multi && p_est <= 0.0 && rq.n_hits <= (uint64_t(1) << 21)) {
             const uint64_t room = std::min<uint64_t>(2 * uint64_t(rq.n_hits), rq.max_sun);
-            if (room > (uint64_t(1) << 20) && batch_buffers(ws, S, room) != cudaSuccess) cudaGetLastError();
+            if (room > (uint64_t(1) << 20) && batch_buffers(ws, S, room) != cudaSuccess) {
+                cudaGetLastError();
+                Scratch &sc = ws;
+                sc.~Scratch();
+                new (&sc) Scratch();
+            }
         }
         while (!done) {
             // plan the next group of batches
@@ -829,6 +832,9 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 CK(ws.scan_parts.ensure(scan_parts(nb) * 4));
                 CK(d_total.ensure(8));
                 CK(d_s_hits.ensure(std::max<uint64_t>(n, 1) * sizeof(HitRec)));
+                CK(d_ecount.ensure(size_t(n_elem0) * 4));
+                CK(d_ecursor.ensure(size_t(n_elem0) * 4));
+                CK(d_etotal.ensure(8));
                 if (rq.records) {
                     // room for this batch's records: its numbered rays at the records per ray seen so far
                     const uint64_t numbered = multi ? global_done : rs.hits_done;

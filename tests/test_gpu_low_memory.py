@@ -36,3 +36,11 @@ def test_a_run_that_found_no_memory_leaves_the_next_one_alone(product):
     want, got = _with_memory_left(product, 20)
     assert want[0] >= 0 and "out of memory" in got[-1]
     assert _run(product) == want
+
+
+@pytest.mark.parametrize("left_mb", [190, 210, 230, 250, 270, 300, 400])
+def test_first_run_with_little_memory_left(product, left_mb):
+    """A context's first run of unknown hit rate reserves its next run's buffers (about 300 MB here);
+    where that room is not to be had, it still gets what it needs itself (about 150 MB)."""
+    want, got = _with_memory_left(product, left_mb)
+    assert want[0] >= 0 and got == want
