@@ -711,11 +711,10 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         cudaEvent_t t_first = new_event(), t_last = new_event();
         CK(cudaEventRecord(t_first, st));
         bool done = false;
-        // what the host reads after queued work -- run state, record count, counters and (small)
-        // accumulators -- in one wait; `fresh` until more work is queued
-        const bool acc_mailed = acc_n <= Workspace::kAccHost;
-        bool fresh = false;
-        auto read_back = [&]() -> cudaError_t {
+        // what the host reads after queued work -- run state, record count, counters and, where the work may
+        // be the run's last, (small) accumulators -- in one wait; `fresh`, `acc_mailed` until more is queued
+        bool fresh = false, acc_mailed = false;
+        auto read_back = [&](bool last) -> cudaError_t {
             cudaError_t e;
             if ((e = cudaEventRecord(t_last, st)) ||
                 (e = cudaMemcpyAsync(&ws.mail->rs, drs, sizeof(RunState), cudaMemcpyDeviceToHost, st)) ||
@@ -726,6 +725,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 if ((e = cudaMemcpyAsync(&ws.mail->nrec, d_rec_count.p, 8, cudaMemcpyDeviceToHost, st))) return e;
                 out.d2h_bytes += 8;
             }
+            acc_mailed = last && acc_n <= Workspace::kAccHost;
             if (acc_mailed && acc_n) {
                 if ((e = cudaMemcpyAsync(ws.acc_host, d_acc.p, acc_n * 8, cudaMemcpyDeviceToHost, st))) return e;
                 out.d2h_bytes += acc_n * 8;
@@ -761,7 +761,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             CK(cudaGetLastError());
             trace_ev.push_back({p1, p2});
             out.batches = 1;
-            CK(read_back());
+            CK(read_back(true));
             const unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
             if (rq.records && rec.overflowed(rec.report(nrec).data(), 1)) continue;
             bool save_over = false;
@@ -926,7 +926,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 out.batches++;
                 fresh = false;
                 if (sync_each) {
-                    CK(read_back());
+                    CK(read_back(queued >= want));
                     rs = ws.mail->rs;
                     const unsigned long long nrec = rq.records ? ws.mail->nrec : 0;
                     const auto report = rec.report(nrec);
@@ -964,7 +964,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
                 if (multi && global_done == rq.n_hits) break;
             }
             if (restart) break;
-            if (!fresh) CK(read_back());
+            if (!fresh) CK(read_back(true));
             rs = ws.mail->rs;
             const uint64_t done_hits = multi ? global_done : rs.hits_done;
             if ((multi ? global_done == rq.n_hits : rs.reached != 0) || out.cancelled ||
@@ -973,7 +973,7 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
             if (!explicit_mode && sun_next > 0) p_est = std::max(double(done_hits) / double(sun_next), 1e-9);
         }
         if (restart) continue;
-        if (!fresh) CK(read_back());  // no batch was needed
+        if (!fresh) CK(read_back(true));  // no batch was needed
         float ms = 0;
         cudaEventElapsedTime(&ms, t_first, t_last);
         out.device_ms = ms;
