@@ -2560,6 +2560,13 @@ static void copy_cols(const ColumnCopy *c, int n, size_t bytes) {
         const size_t at = k % per * kPiece;
         if (q.dst && q.src) memcpy(static_cast<char *>(q.dst) + at, static_cast<const char *>(q.src) + at, std::min(kPiece, bytes - at));
     };
+    // arrays that overlap (a caller that passes one for several columns) are written in column order
+    bool apart = true;
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < i; ++j) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(c[i].dst), b = reinterpret_cast<uintptr_t>(c[j].dst);
+            if (a && b && (a > b ? a - b : b - a) < bytes) apart = false;
+        }
     const size_t nth = std::min<size_t>({pieces, 8, std::max<size_t>(1, std::thread::hardware_concurrency())});
     std::atomic<size_t> next{0};
     auto work = [&]() {
@@ -2567,7 +2574,7 @@ static void copy_cols(const ColumnCopy *c, int n, size_t bytes) {
     };
     std::vector<std::thread> th;
     try {  // fewer helpers where the system gives no more threads
-        if (bytes * size_t(n) >= 4 * kPiece)
+        if (apart && bytes * size_t(n) >= 4 * kPiece)
             for (size_t t = 1; t < nth; ++t) th.emplace_back(work);
     } catch (const std::exception &) {
     }
