@@ -1900,6 +1900,15 @@ bool build_position_frame(const Context *cx, const HostScene &hs, const double s
     SunM sun = cx->sun;
     for (int q = 0; q < 3; ++q) sun.origin[q] = sun_xyz[q];
     out.sun = hs.dev.sun;
+    if (target) {  // before the sun frame, as in build_position: the first error is the one reported
+        Tracker tr;
+        if (!(err = tr.set(sun_xyz, target)).empty()) return false;
+        out.rot.resize(st.elems.size() * 9);
+        for (size_t k = 0; k < st.elems.size(); ++k) {
+            double aim_pt[3];
+            if (!(err = tr.aim(st.elems[k], aim_pt, &out.rot[9 * k])).empty()) return false;
+        }
+    }
     double Rs[9];
     if (!(err = sun_frame(st, sun, out.sun, Rs)).empty()) return false;
     double rmax = 0.0;
@@ -1928,19 +1937,9 @@ bool build_position_frame(const Context *cx, const HostScene &hs, const double s
     g.onx = occ.nx;
     g.ony = occ.ny;
     g.ostride = occ.stride;
-    Tracker tr;
-    if (target) {
-        if (!(err = tr.set(sun_xyz, target)).empty()) return false;
-        out.rot.resize(st.elems.size() * 9);
-    }
     for (size_t k = 0; k < st.elems.size(); ++k) {
         const Elem &e = st.elems[k];
-        const double *R = e.R;
-        if (target) {
-            double aim_pt[3];
-            if (!(err = tr.aim(e, aim_pt, &out.rot[9 * k])).empty()) return false;
-            R = &out.rot[9 * k];
-        }
+        const double *R = target ? &out.rot[9 * k] : e.R;
         if (!e.enabled || !(0.0 <= e.zap) || e.p[0] < 0.0 || e.p[1] < 0.0) continue;
         // |det| of the projected half-axes is their product times the sun's cosine on the plane
         double nz[3];
