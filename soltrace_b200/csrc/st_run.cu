@@ -1501,11 +1501,21 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
     const size_t n_lanes = std::min<size_t>(K, kBatchLanes);
     const uint64_t kMaxBatch = uint64_t(1) << (n_lanes > 1 ? 24 : 26);
     while (ws.lanes.size() + 1 < n_lanes) {
-        ws.lanes.push_back(std::make_unique<Lane>());
-        CK(ws.lanes.back()->create());
+        auto lane = std::make_unique<Lane>();
+        CK(lane->create());
+        ws.lanes.push_back(std::move(lane));
     }
-    for (auto &l : ws.lanes) CK(cudaStreamSynchronize(l->stream));  // idle, unless a run failed
     CK(cudaStreamSynchronize(st));
+    // a batch that ends in an error leaves no lane running: the context's next run copies its tables on
+    // the workspace's own stream, which does not wait for the others
+    struct Drain {
+        std::vector<std::unique_ptr<Lane>> &lanes;
+        bool idle;
+        ~Drain() {
+            for (auto &l : lanes)
+                if (!idle && cudaStreamSynchronize(l->stream) != cudaSuccess) cudaGetLastError();
+        }
+    } drain{ws.lanes, false};
     out.setup_ms = ms_since(t_setup);
 
     size_t ev_used = 0;
@@ -1627,6 +1637,7 @@ bool gpu_run_batch(const HostScene &hs, const std::vector<SunPosition> &pos, con
             }
         }
     }
+    drain.idle = true;
     CK(cudaEventRecord(t_last, st));
     CK(cudaStreamSynchronize(st));
     float ms = 0;
