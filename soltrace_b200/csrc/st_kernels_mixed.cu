@@ -7,11 +7,12 @@ namespace stb {
 template <int FLAT>
 static void resolve(const SceneDev &S, uint64_t s0, const ProbeOut &o, const RunState *rs, cudaStream_t st) {
     // persistent grid: every resident block on every SM
-    static const int per_sm = resident_blocks(k_sun_resolve<1, kResolveMinBlocks, FLAT>, kResolveBlock);
+    constexpr int kBlocks = FLAT ? kResolveFlatMinBlocks : kResolveMinBlocks;
+    static const int per_sm = resident_blocks(k_sun_resolve<1, kBlocks, FLAT>, kResolveBlock);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    k_sun_resolve<1, kResolveMinBlocks, FLAT><<<sms * per_sm, kResolveBlock, 0, st>>>(S, s0, o, rs);
+    k_sun_resolve<1, kBlocks, FLAT><<<sms * per_sm, kResolveBlock, 0, st>>>(S, s0, o, rs);
 }
 int launch_probe_mixed(const SceneDev &S, uint64_t s0, uint32_t n, const ProbeOut &o, const RunState *rs,
                       cudaStream_t st) {

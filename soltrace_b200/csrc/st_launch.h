@@ -22,9 +22,11 @@ constexpr int kFlatWarpBytes = kFlatQueue * (8 + 2) + kFlatHits * 8 + kFlatSeg /
 struct FlatKeys {                   // Philox keys of rounds 4 to 10
     uint32_t k0[7], k1[7];
 };
-// resident blocks per SM asked of the grid probe's element-test kernel (register budget): on the
-// 2,000-heliostat field 2^24 sun rays took 147 us at 6, 142 at 8 and 150 at 4
-constexpr int kResolveMinBlocks = 6;
+// resident blocks per SM asked of the grid probe's element-test kernel (register budget).  Probe of
+// 1e7 hits on the 2,000-heliostat field, double precision: focused (parabolic) heliostats 1.98 ms
+// at 4, 1.93 at 6, 1.89 at 8; round flat ones (kResolveFlatMinBlocks) 1.57, 1.52 and 1.54.  Mixed
+// precision within 0.01 ms of these, but 1.52 for round ones at 8 too.
+constexpr int kResolveMinBlocks = 8, kResolveFlatMinBlocks = 6;
 // resident blocks per SM asked of the trace's shade and search kernels (register budget)
 constexpr int kWfShadeMinBlocks = 4;
 constexpr int kWfSearchMinBlocks = 4;
