@@ -1068,8 +1068,7 @@ __device__ __forceinline__ bool quadric_element(const ElemRec &e) {
 }
 // the hit of a ray on a closed-form element at path length t: point, direction, normal (flipped
 // when hit from behind)
-__device__ __forceinline__ void complete_hit(const ElemRec &e, const double pe[3], const double ce[3],
-                                             const double out[3], double n[3], double t, Hit &h) {
+__device__ __forceinline__ void complete_hit(const double ce[3], const double out[3], double n[3], double t, Hit &h) {
     const int back = (ce[0] * n[0] + ce[1] * n[1] + ce[2] * n[2] < 0) ? 0 : 1;
     for (int q = 0; q < 3; ++q) {
         h.pe[q] = out[q];
@@ -1092,7 +1091,7 @@ __device__ __forceinline__ void closed_hit_at(const ElemRec &e, const double ps[
     element_ray(e, ps, cs, pe, ce);
     point_at(e, pe, ce, t, out);
     if (e.stype != kSurfFlat) quadric_normal(e, out, n);
-    complete_hit(e, pe, ce, out, n, t, h);
+    complete_hit(ce, out, n, t, h);
 }
 
 // CLOSED: the element is known to have a closed-form surface (closed_form_surface), so the
@@ -1136,7 +1135,7 @@ __device__ __forceinline__ bool element_test(const SceneDev &S, const ElemRec &e
     plen = t;
     if (full) {
         if (quadric) quadric_normal(e, out, n);
-        complete_hit(e, pe, ce, out, n, t, *full);
+        complete_hit(ce, out, n, t, *full);
     }
     return true;
 }

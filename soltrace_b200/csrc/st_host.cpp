@@ -1084,8 +1084,6 @@ std::string sun_frame(const StageM &st, SunM &sun, SunDev &sd, double Rs[9]) {
     sun.xmin = 1.0e20;
     sun.ymax = -1.0e20;
     sun.ymin = 1.0e20;
-    const double cd[3] = {0, 0, 1};
-    (void)cd;
     size_t n = 0;
     for (const Elem &e : st.elems) {
         if (!e.enabled) continue;

@@ -12,8 +12,8 @@ constexpr int kResolveBlock = 128;  // threads per block of the grid probe's ele
 constexpr int kCandPerThread = 8;   // sun rays per thread of the grid probe's pre-test kernel
 constexpr int kCandRays = kProbeBlock * kCandPerThread;
 constexpr int kTraceBlock = 128;
-// Probe of flat rectangles (k_sun_probe_flat): 24 warps a block, two blocks a SM (42 registers a
-// thread; 109 KB of shared memory a block with the largest occupancy bitmap)
+// Probe of flat rectangles (k_sun_probe_flat): 24 warps a block, two blocks a SM (40 registers a
+// thread; 110,080 bytes of shared memory a block with the largest occupancy bitmap)
 constexpr int kFlatBlock = 768;
 constexpr int kFlatSeg = 1024;      // sun rays of a warp's segment (32 mask words)
 constexpr int kFlatQueue = 96;      // rays a warp queues for the footprint test (31 + 64, one spare)

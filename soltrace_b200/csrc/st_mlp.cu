@@ -436,8 +436,9 @@ __device__ __forceinline__ void epilogue16(const GemmArgs &g, long long row, int
 // values by 64 K and the products read them transposed in place.  Rows and K beyond the
 // matrices arrive as zeros.
 // Against k_mlp_gemm (one stage, every wait exposed, element loads of transposed operands): the
-// sixteen 256-wide products of a gradient pass over 16,384 rows took 140 us each there and take
-// 17 here (bound by the traffic of their outputs and by filling a single wave of tiles); the
+// sixteen 256-wide products of a gradient pass over 16,384 rows took 140 us each there; here
+// the hidden layers' take 13 to 15 (dX) and 21 (dW): a single wave of 128 tiles whose tensor pipe is
+// active a tenth of the time, the rest being launch, pipeline fill and the outputs' stores.  The
 // pass fell from 2.31 to 0.42 ms.
 constexpr int kPipeThreads = 320;             // warps 0-7 epilogue, 8 loader, 9 products
 constexpr int kPipeBytes = 192 * 1024;        // ring of operand tiles

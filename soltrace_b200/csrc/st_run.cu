@@ -546,8 +546,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
         out.error = "too many flux maps";
         return false;
     }
-    int dev_sms = 148;
-    cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, rq.device);
 
     const int nst = S.n_stages;
     const uint64_t kMaxBatch = uint64_t(1) << 26;
@@ -576,7 +574,6 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
     DevBuf &d_ecount = ws.ecount, &d_ecursor = ws.ecursor, &d_etotal = ws.etotal, &d_s_hits = ws.s_hits;
     RecordRoom<DevBuf> rec(d_recs, sizeof(RecordDev));
     unsigned long long save_cap = 0;
-    (void)dev_sms;
     out.setup_ms = ms_since(t_setup);
 
     double rec_per_ray = 2.0 * nst;  // records per numbered ray expected when sizing the buffer
@@ -1107,8 +1104,8 @@ bool gpu_run(const HostScene &hs, const RunRequest &rq, RunResult &out, Workspac
 // run state, counters and accumulators; its rays draw from the streams of its own seed, so
 // position p's results are those of a single run with that sun and seed.  Positions advance
 // in waves: a wave queues, for every position still short of its hits, the sun rays its hit
-// rate (measured by the previous wave; the first wave probes 2^20 rays) says it needs, with
-// no host round trip inside the wave; the host then reads all positions' run states at once.
+// rate (measured by the previous wave; before the first, the footprints' area over the sun box, or
+// where that is unknown a trial of 2^20 rays) says it needs, with no host round trip inside the wave; the host then reads all positions' run states at once.
 namespace {
 // Where a chunk's positions sit in the device tables (and in a staging area laid out the
 // same way: one region per array, positions end to end).

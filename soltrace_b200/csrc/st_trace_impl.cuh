@@ -674,7 +674,7 @@ static void launch_k_probe(const SceneDev &S, uint64_t s0, uint32_t n, const Pro
 
 // Probe of generated sun rays on a first stage culled by the sun-plane grid, in two
 // kernels so that the double-precision work runs in full warps:
-//   k_sun_candidates (four sun rays per thread, few registers): draws the sun-plane point
+//   k_sun_candidates (eight sun rays per thread, 32 registers): draws the sun-plane point
 //     and runs the float pre-tests of its grid cell; a ray with no passing entry is a miss,
 //     the others are appended to a candidate list;
 //   k_sun_resolve (one thread per listed ray): redraws the point and runs the serial
@@ -759,10 +759,12 @@ __global__ void __launch_bounds__(kResolveBlock) k_sun_resolve_amb(const __grid_
 // Output as k_sun_resolve leaves it: hitting rays listed with their element (a reservation per
 // 64 hits or more), one hit-mask bit per ray, hits per kProbeBlock rays.
 //
-// Bound by the issue of integer instructions in step 1 (about 120 a ray, most of them Philox's
-// products and XORs).  A batch of 2^26 sun rays of the 2,000-heliostat field takes 437 us; one
+// Mostly step 1 (about 120 instructions a ray, most of them Philox's products and XORs).  On 1.6e7 sun
+// rays no unit is full: instruction issue 55 %, the ALU 47 %, the integer-product pipe 46 %; a warp
+// that is not issued waits for table loads (4.3 cycles per issue), shared memory (3.1), a full pipe
+// (1.9) or its own last result (2.2).  A batch of 2^26 sun rays of the 2,000-heliostat field takes 437 us; one
 // thread per ray with the variates converted to double and every ray reading its cell took 620,
-// the double-precision pair k_sun_candidates + k_sun_resolve about 990.  Measured and left: 32
+// the double-precision pair k_sun_candidates + k_sun_resolve about 990.  Measured and left: 16
 // warps an SM more (1024-thread blocks at 32 registers) gave the same time.
 //
 // Philox's first three rounds see a counter whose first word is 0 and whose third and fourth
